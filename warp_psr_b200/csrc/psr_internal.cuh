@@ -346,11 +346,12 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
                             cudaStream_t s, float* ms, V* hist = nullptr, bool rev = false,
                             bool record_increment = false, RelaxDeferred* defer = nullptr);
 
-// Strip-scheduled ordered relaxation (psr_relax.cu): slot-ELL rows in key order, x in key
-// order holds the initial guess and receives the result.
-template <class T, class V>
-void relax_sliced_strips(const int64_t* keys, int64_t rows, int depth, const int32_t* cols, const T* vals,
-                         const V* b, V* x, int iters, cudaStream_t s, float* ms);
+// Strip-scheduled ordered relaxation (psr_relax.cu) of a level in CSR (key order, columns
+// ascending within each row's 27-neighbourhood); x in key order holds the initial guess and
+// receives the result.
+template <class T>
+void relax_sliced_csr(const int64_t* keys, int64_t rows, int depth, const int32_t* offsets, const int32_t* columns,
+                      const T* values, const T* b, T* x, int iters, cudaStream_t s);
 
 // ---------------------------------------------------------------- A11/A12 field.py, reconstruction.py
 template <class T>
