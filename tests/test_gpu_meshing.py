@@ -106,6 +106,25 @@ def test_reconstruction_mesh_fused_matches_callback(dtype, precision):
     assert len(fused.vertices) == fused.metadata["vertices"]
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("shape,slab", [((2, 2, 2), 16), ((9, 17, 33), 16), ((17, 8, 16), 16), ((33, 65, 15), 7),
+                                        ((70, 41, 129), 32), ((129, 130, 131), 1)])
+def test_grids_of_every_spacing_match_pointwise_evaluation(dtype, shape, slab):
+    # from a few nodes per grid (coarser than every cell: nodes evaluated one by one) to several
+    # nodes per finest cell (bricks of nodes from shared functions), odd brick splits among them
+    P, N = _sphere_cloud(3000, dtype, seed=3)
+    res = reconstruct(P, N, depth=5, full_depth=2)
+    bounds = _inner_bounds(P)
+    iso = float(res.evaluate(P)[0].double().mean()) if shape == (2, 2, 2) else res.iso_value
+    fdt = res.field.coefficients.dtype
+    fused = extract_mesh(res, resolution=shape, bounds=bounds, iso_value=iso, slab_size=slab)
+    generic = extract_isosurface(lambda q: (res.evaluate(q)[0] - torch.tensor(iso, dtype=fdt, device="cuda")).contiguous(),
+                                 resolution=shape, bounds=bounds, dtype=fdt)
+    assert torch.equal(fused.indices, generic.indices)
+    assert torch.equal(fused.vertices, generic.vertices)
+    assert fused.metadata["retained_cells"] == generic.metadata["retained_cells"]
+
+
 def test_mesh_vertex_loss_reaches_inputs():
     """loss = sum |v|^2 over the mesh vertices; its gradient on positions and normals against
     central differences (float64, h = 1e-6), with the cell selection and connectivity checked
