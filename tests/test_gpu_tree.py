@@ -1,0 +1,36 @@
+"""The tree built on bitmaps (depths through 11) against the tree built by sorting (PSR_TREE=sort,
+the path of deeper trees): the same support and basis keys, in the same order, for every
+relation of base, full and finest depth."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _cloud(count, seed):
+    rng = np.random.default_rng(seed)
+    n = rng.normal(size=(count, 3))
+    n /= np.linalg.norm(n, axis=1)[:, None]
+    p = n * (1 + 0.2 * n[:, :1]) + 0.05 * rng.normal(size=(count, 3))
+    return torch.from_numpy(p).cuda(), torch.from_numpy(n).cuda()
+
+
+@pytest.mark.parametrize("depth,full_depth,base_depth", [(1, 0, 0), (1, 1, 1), (2, 1, 0), (3, 3, 3), (4, 2, 0),
+                                                         (5, 4, 3), (5, 5, 4), (6, 3, 3), (6, 5, 2), (7, 6, 6),
+                                                         (8, 4, 4), (9, 3, 1), (11, 2, 2)])
+@pytest.mark.parametrize("count", [5, 3000])
+def test_bitmap_tree_has_the_sorted_tree_s_keys(monkeypatch, depth, full_depth, base_depth, count):
+    from warp_psr_b200 import reconstruct
+    P, N = _cloud(count, seed=depth)
+    runs = []
+    for mode in (None, "sort"):
+        if mode:
+            monkeypatch.setenv("PSR_TREE", mode)
+        r = reconstruct(P, N, depth=depth, full_depth=full_depth, base_depth=base_depth, iters=1, scale=1.1)
+        runs.append((r.field.keys.cpu().numpy(), [k.cpu().numpy()
+                                                  for k in r.diagnostics["support_keys"]]))
+    np.testing.assert_array_equal(runs[0][0], runs[1][0])
+    assert len(runs[0][1]) == len(runs[1][1]) == depth + 1
+    for a, b in zip(runs[0][1], runs[1][1]):
+        np.testing.assert_array_equal(a, b)
