@@ -153,7 +153,7 @@ struct DensityData {
   T scale;
   // Kept for the adjoint only (`keep`):
   std::vector<DBuf<int32_t>> parent_of;   // [d]: aggregate index at d-1 of each record at d
-  std::vector<DBuf<int32_t>> splat_order; // [d]: morton order of the depth-d aggregates
+  std::vector<DBuf<int32_t>> splat_order; // [d]: morton order of the aggregates (leaf depth only: the others are in it)
   std::vector<DBuf<int32_t>> splat_slot;  // [d]: unique level value of splat record 27*i+k, or -1
   std::vector<DBuf<T>> level_values;      // [d]: reduced density splat values
   std::vector<HashMap> level_hash;        // [d]: their keys

@@ -164,7 +164,7 @@ __global__ void density_splat_reverse_kernel(const int64_t* keys, const T* value
                                              int d, T scale, const int32_t* slot, const T* g_lvals, T* g_values) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= m) return;
-  const int64_t j = order[i];
+  const int64_t j = order ? order[i] : i;
   int c[3];
   key_coords(keys[j], c);
   const T* v = values + 4 * j;
