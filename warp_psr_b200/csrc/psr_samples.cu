@@ -625,109 +625,125 @@ __global__ void first_keys_kernel(const int32_t* first, int64_t n, uint32_t* key
 
 // normals.py:46-104 — 54 records per group: two 27-node degree-2 splats on the same
 // node `top` (issue #12), weighted by dx and 1-dx.
-// The per-group part of the normal splat: the unit normal times the weight, the splat depth
-// and its two fractions, the cell and the 3 x 3 quadratic B-spline weights.
+// Record keys: the nodes of depth t follow those of the depths below, so the key of node
+// (x, y, z) of depth t is (8^t - 1) / 7 + its index in the depth's grid -- the order of
+// (t, x, y, z), in 31 bits through depth 10 (packed fields take 35 there: 64-bit keys and a
+// radix pass more).  The first key past the deepest level marks a record that is not emitted.
+__host__ __device__ __forceinline__ uint64_t normal_key_base(int t) { return ((uint64_t(1) << (3 * t)) - 1) / 7; }
+
+// The per-group part of the normal splat: the amplitude (unit normal times the weights) of its
+// two splats, the 3 x 3 quadratic B-spline weights, the cell and the splat depth.
 template <class T>
-struct SplatGroup {
-  T nm[3], dx, h, sw;
+struct __align__(16) SplatGroup {
   double b[3][3];
-  int c[3], top, nn, valid, second;
+  T amp[2][3];
+  int c[3], top;  // top -1: the group's mean normal vanishes
+  int second;     // the second splat's records are emitted
 };
 
-// One thread per record (54 per sample): neighbouring threads write neighbouring records.  A
-// block's records span at most six samples; their per-sample values (two divisions and a
-// square root per component, the B-spline weights) are computed once per sample by the
-// block's first threads into shared memory instead of once per record.  Same arithmetic:
-// same records.
-template <class T, class K>
-__global__ void __launch_bounds__(kThreads) normal_splat_kernel(const int32_t* order, int64_t n, const T* sums,
-                                                                const T* nsums, const T* weights, const T* dw,
-                                                                int minimum, int maximum, K* rkeys, int32_t* rids,
-                                                                T* rvals) {
-  constexpr int kGroups = (kThreads + 53) / 54 + 1;  // samples a block's records can touch
-  __shared__ SplatGroup<T> sg[kGroups];
-  const int64_t r0 = blockIdx.x * int64_t(blockDim.x);
-  const int64_t i0 = r0 / 54;
-  if (threadIdx.x < kGroups) {
-    const int64_t i = i0 + threadIdx.x;
-    SplatGroup<T>& G = sg[threadIdx.x];
-    G.valid = 0;
-    if (i < n && i * 54 < r0 + blockDim.x) {
-      int64_t src = order[i];
-      T w = weights[src];
-      T nm[3] = {nsums[3 * src] / w, nsums[3 * src + 1] / w, nsums[3 * src + 2] / w};
-      T length = sqrt(nm[0] * nm[0] + nm[1] * nm[1] + nm[2] * nm[2]);
-      if (length > T(0)) {
-        for (int a = 0; a < 3; ++a) G.nm[a] = nm[a] / length * w;
-        T p[3] = {sums[3 * src] / w, sums[3 * src + 1] / w, sums[3 * src + 2] / w};
-        T depth = dmin(dmax(dw[2 * src], T(minimum)), T(maximum));
-        int top = int(ceil(depth));
-        T dx = T(1.0) - (T(top) - depth);
-        if (top <= minimum) {
-          top = minimum;
-          dx = T(1.0);
-        }
-        if (top > maximum) {
-          top = maximum;
-          dx = T(1.0);
-        }
-        int nn = 1 << top;
-        T h = T(1.0) / T(nn);
-        for (int a = 0; a < 3; ++a) {
-          G.c[a] = ceil_cell(p[a], nn);
-          quadratic(double((p[a] - T(G.c[a]) * h) / h), G.b[a]);
-        }
-        G.top = top;
-        G.nn = nn;
-        G.dx = dx;
-        G.h = h;
-        G.second = fabs(1.0 - double(dx)) > 1e-06;
-        G.sw = dw[2 * src + 1];
-        G.valid = 1;
-      }
+// One thread per group, in the order of the splat (first-index order).
+template <class T>
+__global__ void normal_groups_kernel(const int32_t* __restrict__ order, int64_t n, const T* __restrict__ sums,
+                                     const T* __restrict__ nsums, const T* __restrict__ weights,
+                                     const T* __restrict__ dw, int minimum, int maximum, SplatGroup<T>* groups) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= n) return;
+  SplatGroup<T> G;
+  G.top = -1;
+  G.second = 0;
+  const int64_t src = order[i];
+  const T w = weights[src];
+  const T nm[3] = {nsums[3 * src] / w, nsums[3 * src + 1] / w, nsums[3 * src + 2] / w};
+  const T length = sqrt(nm[0] * nm[0] + nm[1] * nm[1] + nm[2] * nm[2]);
+  if (length > T(0)) {
+    const T p[3] = {sums[3 * src] / w, sums[3 * src + 1] / w, sums[3 * src + 2] / w};
+    const T depth = dmin(dmax(dw[2 * src], T(minimum)), T(maximum));
+    int top = int(ceil(depth));
+    T dx = T(1.0) - (T(top) - depth);
+    if (top <= minimum) {
+      top = minimum;
+      dx = T(1.0);
     }
+    if (top > maximum) {
+      top = maximum;
+      dx = T(1.0);
+    }
+    const int nn = 1 << top;
+    const T h = T(1.0) / T(nn);
+    for (int a = 0; a < 3; ++a) {
+      G.c[a] = ceil_cell(p[a], nn);
+      quadratic(double((p[a] - T(G.c[a]) * h) / h), G.b[a]);
+      const T base = nm[a] / length * w * dw[2 * src + 1] / (h * h * h);
+      G.amp[0][a] = base * dx;
+      G.amp[1][a] = base * (T(1.0) - dx);
+    }
+    G.top = top;
+    G.second = fabs(1.0 - double(dx)) > 1e-06;
   }
-  __syncthreads();
-  const int64_t r = r0 + threadIdx.x;
+  groups[i] = G;
+}
+
+// The records' keys, one thread per record (54 per group, neighbouring threads write neighbouring
+// records).  A record's value is not stored: the reduction makes it again from its group, three
+// products of values that the group's 54 records share in the caches, where 24 bytes (float64)
+// per record written here and gathered back there were most of both kernels' traffic.  Depth 10, 3.5
+// million points: 4,208 us here with the values and 798 us without, 2,249 and 3,188 us there.
+template <class T, class K>
+__global__ void normal_keys_kernel(const SplatGroup<T>* __restrict__ groups, int64_t n, int maximum,
+                                   K* __restrict__ rkeys, int32_t* __restrict__ rids) {
+  const int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (r >= 54 * n) return;
   const int64_t i = r / 54;
-  const int k = int(r % 54);
-  int D = maximum > 0 ? maximum : 1;
-  uint64_t sentinel = uint64_t(1) << (3 * D + 4);
-  rkeys[r] = K(sentinel);
-  rids[r] = int32_t(r);
-  const SplatGroup<T>& G = sg[i - i0];
-  if (!G.valid) return;
-  if (k >= 27 && !G.second) return;
-  T fraction = k < 27 ? G.dx : T(1.0) - G.dx;
-  int q = k % 27;
-  int x = q / 9, y = q / 3 % 3, z = q % 3;
-  int t[3] = {G.c[0] + x - 1, G.c[1] + y - 1, G.c[2] + z - 1};
-  if (dmin(t[0], dmin(t[1], t[2])) >= 0 && dmax(t[0], dmax(t[1], t[2])) < G.nn) {
-    T bw = T(G.b[0][x] * G.b[1][y] * G.b[2][z]);
-    const T h = G.h;
-    rkeys[r] = K((uint64_t(G.top) << (3 * D)) | (uint64_t(t[0]) << (2 * D)) | (uint64_t(t[1]) << D) | uint64_t(t[2]));
-    for (int a = 0; a < 3; ++a) rvals[3 * r + a] = G.nm[a] * G.sw / (h * h * h) * fraction * bw;
+  const int k = int(r % 54), q = k % 27;
+  uint64_t key = normal_key_base(maximum + 1);
+  const SplatGroup<T>& G = groups[i];
+  const int top = G.top;
+  if (top >= 0 && (k < 27 || G.second)) {
+    const int t[3] = {G.c[0] + q / 9 - 1, G.c[1] + q / 3 % 3 - 1, G.c[2] + q % 3 - 1};
+    if (dmin(t[0], dmin(t[1], t[2])) >= 0 && dmax(t[0], dmax(t[1], t[2])) < (1 << top))
+      key = normal_key_base(top) + ((uint64_t(t[0]) << (2 * top)) | (uint64_t(t[1]) << top) | uint64_t(t[2]));
   }
+  rkeys[r] = K(key);
+  rids[r] = int32_t(r);
 }
 
 template <class T, class K>
-__global__ void normal_reduce_kernel(const K* keys, const int32_t* order, const int32_t* heads,
-                                     const int32_t* prefix, int64_t n, const T* values, int D, int64_t* out_keys,
-                                     T* out_values) {
+__global__ void normal_reduce_kernel(const K* __restrict__ keys, const int32_t* __restrict__ order,
+                                     const int32_t* __restrict__ heads, const int32_t* __restrict__ prefix, int64_t n,
+                                     const SplatGroup<T>* __restrict__ groups, int64_t* out_keys, T* out_values) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n || !heads[i]) return;
   int64_t g = prefix[i] - 1;
-  const uint64_t k = keys[i];
+  const K k = keys[i];
   T acc[3] = {T(0), T(0), T(0)};
   for (int64_t j = i; j < n && keys[j] == k; ++j) {
-    int64_t r = order[j];
-    for (int a = 0; a < 3; ++a) acc[a] = acc[a] + values[3 * r + a];
+    const int32_t r = order[j];
+    const SplatGroup<T>& G = groups[r / 54];
+    const int e = r % 54, q = e % 27;
+    const T bw = T(G.b[0][q / 9] * G.b[1][q / 3 % 3] * G.b[2][q % 3]);
+    for (int a = 0; a < 3; ++a) acc[a] = acc[a] + G.amp[e / 27][a] * bw;
   }
-  uint64_t mask = (uint64_t(1) << D) - 1;
-  out_keys[g] = basis_key(int(k >> (3 * D)), int((k >> (2 * D)) & mask), int((k >> D) & mask), int(k & mask));
+  const int t = (63 - __clzll((long long)(7 * uint64_t(k) + 1))) / 3;
+  const uint64_t at = uint64_t(k) - normal_key_base(t), mask = (uint64_t(1) << t) - 1;
+  out_keys[g] = basis_key(t, int((at >> (2 * t)) & mask), int((at >> t) & mask), int(at & mask));
   for (int a = 0; a < 3; ++a) out_values[4 * g + a] = -acc[a];  // normals.py:106-110,219-221
   out_values[4 * g + 3] = -T(0);
+}
+
+// offsets[d]: unique records of the depths below d, from the sorted keys and their head counts.
+template <class K>
+__global__ void normal_offsets_kernel(const K* keys, const int32_t* prefix, int64_t n, int levels, int64_t* offsets) {
+  const int d = threadIdx.x;
+  if (d >= levels) return;
+  int64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) / 2;
+    if (uint64_t(keys[mid]) < normal_key_base(d))
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  offsets[d] = lo ? prefix[lo - 1] : 0;
 }
 
 // normals.py:132-147 contributions (raw depth * w, splat weight * w, w) in first-index
@@ -795,20 +811,6 @@ __global__ void __launch_bounds__(kAverageThreads) average_finish_kernel(const T
   }
 }
 
-__global__ void depth_offsets_kernel(const int64_t* keys, int64_t n, int levels, int64_t* offsets) {
-  int d = threadIdx.x;
-  if (d >= levels) return;
-  int64_t target = int64_t(d) << 48, lo = 0, hi = n;
-  while (lo < hi) {
-    int64_t mid = (lo + hi) / 2;
-    if (keys[mid] < target)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  offsets[d] = lo;
-}
-
 template <class T>
 NormalData<T> build_normals(const SampleGroups<T>& g, const DensityData<T>& D, int minimum, int maximum,
                             cudaStream_t s, bool keep) {
@@ -820,36 +822,40 @@ NormalData<T> build_normals(const SampleGroups<T>& g, const DensityData<T>& D, i
   PSR_LAUNCH_CHECK();
   sort_pairs(fk.p, sfk.p, ids.p, order.p, n, 32, s);
   int64_t r = 54 * n;
-  int Db = maximum > 0 ? maximum : 1;
   {
+    DBuf<SplatGroup<T>> groups(n, s);
+    normal_groups_kernel<T><<<blocks_for(n, 128), 128, 0, s>>>(order.p, n, g.sums.p, g.normal_sums.p, g.weights.p,
+                                                              D.dw.p, minimum, maximum, groups.p);
+    PSR_LAUNCH_CHECK();
     DBuf<int32_t> rids(r, s), rorder(r, s);
-    DBuf<T> rvals(3 * r, s);
-    // Record keys of 3 Db + 5 bits: 32-bit keys up to depth 9 (a third less data through the
-    // sort's passes), else 64-bit.  Same keys, same stable order either way.
+    const uint64_t sentinel = normal_key_base(maximum + 1);
     auto splat_reduce = [&](auto key_tag) {
       using K = decltype(key_tag);
       DBuf<K> rkeys(r, s), skeys(r, s);
-      normal_splat_kernel<T, K><<<blocks_for(54 * n), kThreads, 0, s>>>(order.p, n, g.sums.p, g.normal_sums.p,
-                                                                        g.weights.p, D.dw.p, minimum, maximum,
-                                                                        rkeys.p, rids.p, rvals.p);
+      normal_keys_kernel<T, K><<<blocks_for(r), kThreads, 0, s>>>(groups.p, n, maximum, rkeys.p, rids.p);
       PSR_LAUNCH_CHECK();
-      sort_pairs(rkeys.p, skeys.p, rids.p, rorder.p, r, 3 * Db + 5, s);
+      sort_pairs(rkeys.p, skeys.p, rids.p, rorder.p, r, bits_for(sentinel), s);
       DBuf<int32_t> heads, prefix;
-      int64_t u = segment_heads(skeys.p, r, uint64_t(1) << (3 * Db + 4), 0, heads, prefix, s);
+      mark_segments(skeys.p, r, sentinel, 0, heads, prefix, s);
+      DBuf<int64_t> off(maximum + 2, s);
+      normal_offsets_kernel<K><<<1, 32, 0, s>>>(skeys.p, prefix.p, r, maximum + 2, off.p);
+      PSR_LAUNCH_CHECK();
+      N.offsets = read_vector(off.p, maximum + 2, s);
+      const int64_t u = N.offsets.back();
       N.count = u;
       N.keys.alloc(u, s);
       N.values.alloc(4 * u, s);
-      normal_reduce_kernel<T, K><<<blocks_for(r), kThreads, 0, s>>>(skeys.p, rorder.p, heads.p, prefix.p, r,
-                                                                    rvals.p, Db, N.keys.p, N.values.p);
+      normal_reduce_kernel<T, K><<<blocks_for(r), kThreads, 0, s>>>(skeys.p, rorder.p, heads.p, prefix.p, r, groups.p,
+                                                                    N.keys.p, N.values.p);
       PSR_LAUNCH_CHECK();
       if (keep) {
         N.record_slot.alloc(r, s);
-        segment_slot_kernel<<<blocks_for(r), kThreads, 0, s>>>(rorder.p, prefix.p, skeys.p, r,
-                                                               uint64_t(1) << (3 * Db + 4), 0, N.record_slot.p);
+        segment_slot_kernel<<<blocks_for(r), kThreads, 0, s>>>(rorder.p, prefix.p, skeys.p, r, sentinel, 0,
+                                                               N.record_slot.p);
         PSR_LAUNCH_CHECK();
       }
     };
-    if (3 * Db + 5 <= 32)
+    if (sentinel <= 0xffffffffu)
       splat_reduce(uint32_t());
     else
       splat_reduce(uint64_t());
@@ -864,10 +870,6 @@ NormalData<T> build_normals(const SampleGroups<T>& g, const DensityData<T>& D, i
   N.average.alloc(3, s);
   average_finish_kernel<T><<<1, kAverageThreads, 0, s>>>(partial.p, chunks, N.average.p);
   PSR_LAUNCH_CHECK();
-  DBuf<int64_t> off(maximum + 2, s);
-  depth_offsets_kernel<<<1, 32, 0, s>>>(N.keys.p, N.count, maximum + 2, off.p);
-  PSR_LAUNCH_CHECK();
-  N.offsets = read_vector(off.p, maximum + 2, s);
   if (keep) N.group_order = std::move(order);
   return N;
 }
