@@ -329,6 +329,25 @@ struct StripSchedule {
 };
 void build_strip_schedule(const int64_t* keys, int64_t rows, int depth, StripSchedule& S, cudaStream_t s);
 
+// How a level's sweeps are cut into tasks: strips per slice, their descriptions and the shared
+// memory a task takes.  Depends on the schedule, the sweeps, the types and the direction only, so
+// it can be made before the level's right-hand side is known.
+struct StripPlan {
+  int strips = 0, unstaged = 0, nvisits = 0, cap = 0, row_cap = 0, b_cap = 0;
+  int64_t smem = 0;
+  DBuf<int32_t> xstart, bounds;
+  DBuf<int2> visits;
+  DBuf<char> meta;
+};
+template <class T, class V, class I>
+void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cudaStream_t s);
+
+// relax_strips_scheduled (below) with its plan at hand.
+template <class T, class V, class I>
+void relax_strips_planned(const StripSchedule& S, const StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
+                          int iters, cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment,
+                          RelaxDeferred* defer);
+
 // Strip-scheduled relaxation of operator rows already in schedule order: values T[28] and
 // group-relative neighbour indices I[32] per row, b with 16 bytes of slack; x in key order
 // holds the initial guess and receives the result.

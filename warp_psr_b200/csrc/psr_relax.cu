@@ -1542,29 +1542,17 @@ static bool relax_pipeline(const StripSchedule& S, const T* svals, const I* sidx
 }
 
 template <class T, class V, class I>
-void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sidx, const V* sb, V* x, int iters,
-                            cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment, RelaxDeferred* defer) {
+void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cudaStream_t s) {
   const int64_t rows = S.rows;
   if (iters <= 0 || rows <= 0) return;
-  const int depth = S.depth;
-  const int n = 1 << depth;
+  const int n = 1 << S.depth;
   const int nx = n + 2;
   const int per16 = 16 / int(sizeof(V));
-  const int32_t* perm = S.perm.p;
   const int32_t* off = S.off.p;
-  DBuf<V> x0(rows + 16, s), x1(rows + 16, s);  // slack: 16-byte copies may read past the last row
-  gather_x_kernel<V><<<blocks_for(rows), kThreads, 0, s>>>(perm, rows, x, x1.p);
+  P.xstart.alloc(int64_t(n + 1) * 4 * nx, s);
+  DBuf<int32_t>& xstart = P.xstart;
+  xstart_kernel<<<blocks_for(int64_t(n + 1) * 4 * nx), kThreads, 0, s>>>(S.skeys.p, off, n, xstart.p);
   PSR_LAUNCH_CHECK();
-  const int64_t* skeys_p = S.skeys.p;
-  DBuf<int32_t> xstart(int64_t(n + 1) * 4 * nx, s);
-  xstart_kernel<<<blocks_for(int64_t(n + 1) * 4 * nx), kThreads, 0, s>>>(skeys_p, off, n, xstart.p);
-  PSR_LAUNCH_CHECK();
-  if (relax_pipeline<T, V, I>(S, svals, sidx, sb, xstart.p, x0.p, x1.p, iters, s, ms, hist, rev, record_increment,
-                              defer)) {
-    scatter_back_kernel<V><<<blocks_for(rows), kThreads, 0, s>>>(perm, rows, ((iters - 1) & 1) ? x1.p : x0.p, x);
-    PSR_LAUNCH_CHECK();
-    return;
-  }
   // Strips per slice: a wave (iters x strips tasks) fills about seven eighths of the persistent
   // grid, leaving CTAs that take the next wave's tasks early and prefetch their operator rows;
   // at least ~128 rows per strip.  More strips are taken (up to twice as many) while more than
@@ -1585,11 +1573,8 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
     }
   }
   const int base_strips = strips;
-  DBuf<int> ctrl(3 * 32, s);  // task counter, error word, capacities: one 128-byte line each
-  int* counter = ctrl.p;
-  int* error = ctrl.p + 32;
-  int* caps_dev = ctrl.p + 64;
-  DBuf<int32_t> bounds;
+  DBuf<int> caps_dev(4, s);
+  DBuf<int32_t>& bounds = P.bounds;
   std::vector<int> caps;
   // 16-bit index rows reach the footprint through offsets below 2^15 (idx_absent).
   // PSR_RELAX_FOOTPRINT_LIMIT lowers that bound (test override: the strip narrowing below,
@@ -1615,15 +1600,15 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
     strip_bounds_kernel<<<blocks_for(int64_t(n + 1) * (strips + 1)), kThreads, 0, s>>>(xstart.p, n, strips,
                                                                                         bounds.p);
     PSR_LAUNCH_CHECK();
-    ctrl.zero();
+    caps_dev.zero();
     footprint_kernel<<<blocks_for((n + 1) * strips), kThreads, 0, s>>>(xstart.p, bounds.p, n, strips, per16,
-                                                                        rev ? 1 : 0, caps_dev);
+                                                                        rev ? 1 : 0, caps_dev.p);
     PSR_LAUNCH_CHECK();
     unstaged_kernel<<<blocks_for((n + 1) * strips), kThreads, 0, s>>>(xstart.p, bounds.p, n, strips, per16,
                                                                        rev ? 1 : 0, budget, int(row_bytes),
-                                                                       int(sizeof(V)), caps_dev);
+                                                                       int(sizeof(V)), caps_dev.p);
     PSR_LAUNCH_CHECK();
-    caps = read_vector(caps_dev, 4, s);  // footprint, rows, right-hand side, unstaged tasks
+    caps = read_vector(caps_dev.p, 4, s);  // footprint, rows, right-hand side, unstaged tasks
     // narrow the strips until the largest footprint fits the 16-bit offsets
     if (!(sizeof(I) == 4 || caps[0] <= fp_limit) && strips < 256) {
       strips = std::min(256, 2 * strips);
@@ -1647,23 +1632,70 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
     int first = std::max(0, (q - n + 1) / 2), last = std::min(iters - 1, q / 2);
     for (int t = first; t <= last; ++t) visits.push_back(make_int2(n - q + 2 * t, t));
   }
-  DBuf<int2> dvisits(int64_t(visits.size()), s);
-  PSR_CUDA(cudaMemcpyAsync(dvisits.p, visits.data(), visits.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+  P.nvisits = int(visits.size());
+  P.visits.alloc(P.nvisits, s);
+  PSR_CUDA(cudaMemcpyAsync(P.visits.p, visits.data(), visits.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+  // Shared memory: the footprint, plus the staged rows of tasks that fit.
+  const int64_t fp_bytes = fp_bytes_of(maxfp);
+  if (fp_bytes > budget) throw Error(4, "ordered relaxation: a strip footprint exceeds shared memory");
+  P.strips = strips;
+  P.unstaged = caps[3];
+  P.cap = std::max(maxfp, 1);
+  int64_t rc = row_capacity(maxfp, maxrows, maxb).first;
+  // PSR_RELAX_ROW_CAP caps the staged rows per task (test override: 0 sends every task down
+  // the global-memory row path that only tasks too large for shared memory take).
+  if (const char* env = std::getenv("PSR_RELAX_ROW_CAP")) {
+    const int forced = std::atoi(env);
+    if (forced >= 0) rc = std::min<int64_t>(rc, forced);
+  }
+  P.row_cap = int(rc);
+  P.b_cap = int(std::min<int64_t>(maxb, rc + 4 * per16) / per16 * per16);
+  P.smem = std::max<int64_t>(16, fp_bytes + rc * (kSlotsR * int64_t(sizeof(T)) + kIdxSlots * int64_t(sizeof(I))) +
+                                     ((int64_t(P.b_cap) * int64_t(sizeof(V)) + 15) & ~int64_t(15)));
+  P.meta.alloc(int64_t(n + 1) * strips * int64_t(sizeof(StripMeta)), s);
+  auto mk = rev ? strip_meta_kernel<true> : strip_meta_kernel<false>;
+  mk<<<blocks_for(int64_t(n + 1) * strips, 128), 128, 0, s>>>(xstart.p, bounds.p, off, n, strips, per16, P.cap,
+                                                               P.row_cap, P.b_cap, int(row_bytes), int(sizeof(V)),
+                                                               reinterpret_cast<StripMeta*>(P.meta.p));
+  PSR_LAUNCH_CHECK();
+}
+
+template <class T, class V, class I>
+void relax_strips_planned(const StripSchedule& S, const StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
+                          int iters, cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment,
+                          RelaxDeferred* defer) {
+  const int64_t rows = S.rows;
+  if (iters <= 0 || rows <= 0) return;
+  const int depth = S.depth;
+  const int n = 1 << depth;
+  const int32_t* perm = S.perm.p;
+  DBuf<V> x0(rows + 16, s), x1(rows + 16, s);  // slack: 16-byte copies may read past the last row
+  gather_x_kernel<V><<<blocks_for(rows), kThreads, 0, s>>>(perm, rows, x, x1.p);
+  PSR_LAUNCH_CHECK();
+  if (relax_pipeline<T, V, I>(S, svals, sidx, sb, P.xstart.p, x0.p, x1.p, iters, s, ms, hist, rev, record_increment,
+                              defer)) {
+    scatter_back_kernel<V><<<blocks_for(rows), kThreads, 0, s>>>(perm, rows, ((iters - 1) & 1) ? x1.p : x0.p, x);
+    PSR_LAUNCH_CHECK();
+    return;
+  }
+  const int strips = P.strips;
+  DBuf<int> ctrl(2 * 32, s);  // task counter and error word: one 128-byte line each
+  ctrl.zero();
   StripLevel L{};
   L.n = n;
   L.strips = strips;
-  L.nvisits = int(visits.size());
+  L.nvisits = P.nvisits;
   L.vals = svals;
   L.nidx = sidx;
   L.b = sb;
   L.xb0 = x0.p;
   L.xb1 = x1.p;
-  L.visits = dvisits.p;
+  L.visits = P.visits.p;
   DBuf<int> done(int64_t(n + 1) * strips * kFlagPad, s);
   done.zero();
   L.done = done.p;
-  L.counter = counter;
-  L.error = error;
+  L.counter = ctrl.p;
+  L.error = ctrl.p + 32;
   L.hist = hist;
   L.rows = rows;
   L.iters = iters;
@@ -1677,35 +1709,17 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
       L.stall = 1;
       L.poll_log2 = 12;
     }
-  // Shared memory: the footprint, plus the staged rows of tasks that fit.
-  const int64_t fp_bytes = fp_bytes_of(maxfp);
-  if (fp_bytes > budget) throw Error(4, "ordered relaxation: a strip footprint exceeds shared memory");
-  L.cap = std::max(maxfp, 1);
-  int64_t rc = row_capacity(maxfp, maxrows, maxb).first;
-  // PSR_RELAX_ROW_CAP caps the staged rows per task (test override: 0 sends every task down
-  // the global-memory row path that only tasks too large for shared memory take).
-  if (const char* env = std::getenv("PSR_RELAX_ROW_CAP")) {
-    const int forced = std::atoi(env);
-    if (forced >= 0) rc = std::min<int64_t>(rc, forced);
-  }
-  L.row_cap = int(rc);
-  L.b_cap = int(std::min<int64_t>(maxb, rc + 4 * per16) / per16 * per16);
-  int64_t smem = fp_bytes + rc * (kSlotsR * int64_t(sizeof(T)) + kIdxSlots * int64_t(sizeof(I))) +
-                 ((int64_t(L.b_cap) * int64_t(sizeof(V)) + 15) & ~int64_t(15));
-  smem = std::max<int64_t>(smem, 16);
-  DBuf<StripMeta> meta(int64_t(n + 1) * strips, s);
-  {
-    auto mk = rev ? strip_meta_kernel<true> : strip_meta_kernel<false>;
-    mk<<<blocks_for(int64_t(n + 1) * strips, 128), 128, 0, s>>>(xstart.p, bounds.p, off, n, strips, per16, L.cap,
-                                                                 L.row_cap, L.b_cap, int(row_bytes), int(sizeof(V)),
-                                                                 meta.p);
-    PSR_LAUNCH_CHECK();
-  }
-  L.meta = meta.p;
+  L.cap = P.cap;
+  L.row_cap = P.row_cap;
+  L.b_cap = P.b_cap;
+  L.meta = reinterpret_cast<const StripMeta*>(P.meta.p);
+  const int64_t smem = P.smem;
   auto kernel = rev ? strip_gs_kernel<T, V, I, true> : strip_gs_kernel<T, V, I, false>;
   PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  const int64_t total_tasks = int64_t(visits.size()) * strips;
-  const int grid = int(std::min<int64_t>(total_tasks, ctas));
+  const int64_t total_tasks = int64_t(P.nvisits) * strips;
+  // a wave's tasks and the next one's, whose rows are fetched ahead: a coarse level leaves the
+  // other SMs to the preparation of the finer ones
+  const int grid = int(std::min<int64_t>({total_tasks, int64_t(kRelaxCtasPerSm) * device_sms(), 2ll * strips * iters}));
   const char* trace_file = std::getenv("PSR_RELAX_TRACE_FILE");
   DBuf<long long> trace;
   if (trace_file) {
@@ -1750,14 +1764,23 @@ void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sid
   if (trace_file) {
     std::vector<long long> h = read_vector(trace.p, total_tasks * kTraceSlots, s);
     if (FILE* f = std::fopen(trace_file, "ab")) {
-      long long header[8] = {depth, n, strips, L.row_cap, grid, total_tasks, caps[3], kTraceSlots};
+      long long header[8] = {depth, n, strips, L.row_cap, grid, total_tasks, P.unstaged, kTraceSlots};
       std::fwrite(header, sizeof(header), 1, f);
+      const std::vector<int2> visits = read_vector(P.visits.p, P.nvisits, s);
       std::fwrite(visits.data(), sizeof(int2), visits.size(), f);
       std::fwrite(h.data(), sizeof(long long), h.size(), f);
       std::fclose(f);
     }
   }
   throw_relax_error(err);
+}
+
+template <class T, class V, class I>
+void relax_strips_scheduled(const StripSchedule& S, const T* svals, const I* sidx, const V* sb, V* x, int iters,
+                            cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment, RelaxDeferred* defer) {
+  StripPlan P;
+  plan_strips<T, V, I>(S, iters, rev, P, s);
+  relax_strips_planned<T, V, I>(S, P, svals, sidx, sb, x, iters, s, ms, hist, rev, record_increment, defer);
 }
 
 void build_strip_schedule(const int64_t* keys, int64_t rows, int depth, StripSchedule& S, cudaStream_t s) {
@@ -1844,6 +1867,10 @@ template void relax_sliced_csr<double>(const int64_t*, int64_t, int, const int32
 
 namespace psr {
 #define PSR_SCHED(T, V, I)                                                                                       \
+  template void plan_strips<T, V, I>(const StripSchedule&, int, bool, StripPlan&, cudaStream_t);                 \
+  template void relax_strips_planned<T, V, I>(const StripSchedule&, const StripPlan&, const T*, const I*,        \
+                                              const V*, V*, int, cudaStream_t, float*, V*, bool, bool,           \
+                                              RelaxDeferred*);                                                   \
   template void relax_strips_scheduled<T, V, I>(const StripSchedule&, const T*, const I*, const V*, V*, int,  \
                                                 cudaStream_t, float*, V*, bool, bool, RelaxDeferred*);
 PSR_SCHED(float, float, int16_t)

@@ -1493,6 +1493,81 @@ static PointsData<T> make_points(const DensityData<T>& D, const NormalData<T>& N
   return P;
 }
 
+// A stream for work beside the caller's: begins after what the caller's stream holds when it is
+// first asked for, and the caller's stream waits for all of it before the stream goes.
+struct SideStream {
+  cudaStream_t main = nullptr, side = nullptr;
+  explicit SideStream(cudaStream_t s) : main(s) {}
+  SideStream(const SideStream&) = delete;
+  SideStream& operator=(const SideStream&) = delete;
+  static void order(cudaStream_t first, cudaStream_t then) {
+    cudaEvent_t e = nullptr;
+    PSR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const cudaError_t recorded = cudaEventRecord(e, first);
+    const cudaError_t waited = recorded == cudaSuccess ? cudaStreamWaitEvent(then, e, 0) : recorded;
+    cudaEventDestroy(e);
+    PSR_CUDA(waited);
+  }
+  cudaStream_t get() {
+    if (!side) {
+      PSR_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+      order(main, side);
+    }
+    return side;
+  }
+  ~SideStream() {
+    if (!side) return;
+    try {
+      order(side, main);
+    } catch (...) {
+      cudaStreamSynchronize(side);
+    }
+    cudaStreamDestroy(side);
+  }
+};
+
+// One level's point constraints, operator rows, schedule and sweep plan, before the chain takes
+// them.
+template <class T>
+struct LevelPrep {
+  PointsData<T> P;
+  DBuf<int32_t> cols;
+  DBuf<T> vals, b;
+  StripSchedule sched;
+  StripPlan plan;
+  DBuf<char> svals, sidx;
+  DBuf<int2> cell_ranges;
+  cudaEvent_t ready = nullptr;  // recorded on the side stream after the preparation
+  // From here on the buffers belong to stream s (it waits for the preparation): they are used and
+  // freed in its order.
+  void hand_over(cudaStream_t s) {
+    if (!ready) return;
+    PSR_CUDA(cudaStreamWaitEvent(s, ready, 0));
+    auto take = [s](auto&... buffer) { ((buffer.s = s), ...); };
+    take(P.pos, P.w, P.spos, P.sw, P.ids, P.bstart, P.bkeys, P.bins.slots, cols, vals, b, sched.perm, sched.inv,
+         sched.off, sched.skeys, plan.xstart, plan.bounds, plan.visits, plan.meta, svals, sidx, cell_ranges);
+  }
+  void release() { *this = LevelPrep(); }
+  LevelPrep() = default;
+  LevelPrep(LevelPrep&& o) noexcept { *this = std::move(o); }
+  LevelPrep& operator=(LevelPrep&& o) noexcept {
+    P = std::move(o.P);
+    cols = std::move(o.cols);
+    vals = std::move(o.vals);
+    b = std::move(o.b);
+    sched = std::move(o.sched);
+    plan = std::move(o.plan);
+    svals = std::move(o.svals);
+    sidx = std::move(o.sidx);
+    cell_ranges = std::move(o.cell_ranges);
+    std::swap(ready, o.ready);
+    return *this;
+  }
+  ~LevelPrep() {
+    if (ready) cudaEventDestroy(ready);
+  }
+};
+
 template <class T>
 void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalData<T>& N,
                   const std::vector<int64_t>& level_offsets, const int64_t* all_keys, const HashMap& all_hash,
@@ -1619,65 +1694,65 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
     tp->screened = screened;
     tp->mixed = sizeof(T) == 8 && p.precision == 1;
   }
-  DBuf<T> cumulative;
-  for (int d = base; d <= p.solve_depth; ++d) {
-    int64_t n = count_at(d);
-    if (!n) break;
-    if (tp) tp->top = d;
-    PointsData<T> P;
-    if (screened) P = make_points(D, N, bh, d, p.point_weight, bool(p.exact), s);
-    PointsView<T> pv = screened ? P.view() : PointsView<T>();
-    int res = 1 << d;
-    DBuf<double> table(int64_t(res + 1) * 6, s);
-    stiffness_table_kernel<<<blocks_for(res + 1), kThreads, 0, s>>>(d, d, table.p);
+  const bool mixed = sizeof(T) == 8 && p.precision == 1;
+  // Point constraints, operators, schedules and sweep plans depend on no level's solution, only
+  // the chain base solve -> (cross term, sweeps, prolongation) per level does, and its coarse end
+  // leaves most of the GPU idle: the base solve runs on one CTA and the sweeps of the coarse
+  // levels on a few dozen.  So the finer levels are prepared on a stream of their own while the
+  // chain starts (a depth-8 float32 call 8.17 -> 7.48 ms, depth-9 mixed
+  // 20.7 -> 20.0 ms, 2,011 points at depth 5 2.60 -> 2.42 ms).  What a
+  // level's preparation allocates belongs to that stream until the chain has waited for the
+  // level, and to the caller's stream from then on (LevelPrep::hand_over).
+  SideStream side(s);  // outlives what is prepared on it
+  std::vector<LevelPrep<T>> prepared(finest + 1);
+  const bool finer = p.solve_depth > base && count_at(base) > 0 && count_at(base + 1) > 0;
+  const cudaStream_t q_finer = finer ? side.get() : s;
+  auto prepare = [&](int d, cudaStream_t q) {
+    const int64_t n = count_at(d);
+    LevelPrep<T>& L = prepared[d];
+    if (screened) L.P = make_points(D, N, bh, d, p.point_weight, bool(p.exact), q);
+    const PointsView<T> pv = screened ? L.P.view() : PointsView<T>();
+    const int res = 1 << d;
+    DBuf<double> table(int64_t(res + 1) * 6, q);
+    stiffness_table_kernel<<<blocks_for(res + 1), kThreads, 0, q>>>(d, d, table.p);
     PSR_LAUNCH_CHECK();
     // The base level keeps key-order rows for its multigrid; finer levels are assembled
     // straight into the schedule order of the strip-scheduled relaxation.
-    const bool sliced = d > base;
-    const bool mixed = sizeof(T) == 8 && p.precision == 1;
-    DBuf<int32_t> cols;
-    DBuf<T> vals, b;
-    StripSchedule sched;
-    DBuf<char> svals, sidx;
-    DBuf<int2> cell_ranges;  // the screening cells' point ranges of each row, assembly -> cross term
-    if (!sliced) {
-      cols.alloc(kSlots * n, s);
-      vals.alloc(kSlots * n, s);
-      b.alloc(n, s);
-      if (screened)
-        assemble_level_kernel<T, true><<<blocks_for(n, 128), 128, 0, s>>>(keys_at(d), n, d, bcv, level_offsets[d],
-                                                                           table.p, pv, loads[d].p, cols.p, vals.p,
-                                                                           b.p);
-      else
-        assemble_level_kernel<T, false><<<blocks_for(n, 128), 128, 0, s>>>(keys_at(d), n, d, bcv, level_offsets[d],
-                                                                            table.p, pv, loads[d].p, cols.p, vals.p,
-                                                                            b.p);
+    if (d == base) {
+      L.cols.alloc(kSlots * n, q);
+      L.vals.alloc(kSlots * n, q);
+      L.b.alloc(n, q);
+      auto assemble = screened ? assemble_level_kernel<T, true> : assemble_level_kernel<T, false>;
+      assemble<<<blocks_for(n, 128), 128, 0, q>>>(keys_at(d), n, d, bcv, level_offsets[d], table.p, pv, loads[d].p,
+                                                  L.cols.p, L.vals.p, L.b.p);
       PSR_LAUNCH_CHECK();
     } else {
-      build_strip_schedule(keys_at(d), n, d, sched, s);
-      if (screened) cell_ranges.alloc(8 * n, s);
+      StripSchedule& sched = L.sched;
+      build_strip_schedule(keys_at(d), n, d, sched, q);
+      if (screened) L.cell_ranges.alloc(8 * n, q);
       const int sbytes = mixed ? 4 : int(sizeof(T));
       const int ibytes = sched.wide ? 4 : 2;
-      svals.alloc(kSlots * n * sbytes, s);
-      sidx.alloc(32 * n * ibytes, s);
-      b.alloc(n + 4, s);
-      b.zero();
+      L.svals.alloc(kSlots * n * sbytes, q);
+      L.sidx.alloc(32 * n * ibytes, q);
+      L.b.alloc(n + 4, q);
+      L.b.zero();
       auto launch = [&](auto s_tag, auto i_tag) {
         using S = decltype(s_tag);
         using I = decltype(i_tag);
-        S* sv = reinterpret_cast<S*>(svals.p);
-        I* si = reinterpret_cast<I*>(sidx.p);
+        S* sv = reinterpret_cast<S*>(L.svals.p);
+        I* si = reinterpret_cast<I*>(L.sidx.p);
         // key, float64 load, schedule position, operator row, index row, b, screening cell ranges
         const double row_bytes = 8 + 8 + 4 + kSlots * sizeof(S) + 32 * sizeof(I) + sizeof(T) + (screened ? 64 : 0);
-        KernelClock clock(kClkAssembleSliced, n * row_bytes + (screened ? P.m * 4.0 * sizeof(T) : 0.0), double(n), s);
-        if (screened)
-          assemble_sliced_kernel<T, S, I, true><<<blocks_for(n, 128), 128, 0, s>>>(
-              keys_at(d), n, d, bcv, level_offsets[d], table.p, pv, loads[d].p, sched.inv.p, sched.off.p, sv, si, b.p,
-              cell_ranges.p);
-        else
-          assemble_sliced_kernel<T, S, I, false><<<blocks_for(n, 128), 128, 0, s>>>(
-              keys_at(d), n, d, bcv, level_offsets[d], table.p, pv, loads[d].p, sched.inv.p, sched.off.p, sv, si, b.p);
-        PSR_LAUNCH_CHECK();
+        {
+          KernelClock clock(kClkAssembleSliced, n * row_bytes + (screened ? L.P.m * 4.0 * sizeof(T) : 0.0), double(n),
+                            q);
+          auto assemble = screened ? assemble_sliced_kernel<T, S, I, true> : assemble_sliced_kernel<T, S, I, false>;
+          assemble<<<blocks_for(n, 128), 128, 0, q>>>(keys_at(d), n, d, bcv, level_offsets[d], table.p, pv,
+                                                      loads[d].p, sched.inv.p, sched.off.p, sv, si, L.b.p,
+                                                      L.cell_ranges.p);
+          PSR_LAUNCH_CHECK();
+        }
+        plan_strips<S, T, I>(sched, p.iters, false, L.plan, q);
       };
       if (mixed) {
         if (sched.wide)
@@ -1691,6 +1766,30 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
           launch(T(), int16_t());
       }
     }
+    if (q != s) {
+      PSR_CUDA(cudaEventCreateWithFlags(&L.ready, cudaEventDisableTiming));
+      PSR_CUDA(cudaEventRecord(L.ready, q));
+    }
+  };
+  DBuf<T> cumulative;
+  for (int d = base; d <= p.solve_depth; ++d) {
+    int64_t n = count_at(d);
+    if (!n) break;
+    if (tp) tp->top = d;
+    if (d == base)
+      prepare(d, s);
+    else if (d == base + 1)  // the base solve is under way on s
+      for (int e = d; e <= p.solve_depth && count_at(e); ++e) prepare(e, q_finer);
+    LevelPrep<T>& L = prepared[d];
+    L.hand_over(s);
+    PointsData<T>& P = L.P;
+    const PointsView<T> pv = screened ? P.view() : PointsView<T>();
+    const int res = 1 << d;
+    DBuf<int32_t>& cols = L.cols;
+    DBuf<T>&vals = L.vals, &b = L.b;
+    StripSchedule& sched = L.sched;
+    DBuf<char>&svals = L.svals, &sidx = L.sidx;
+    DBuf<int2>& cell_ranges = L.cell_ranges;  // the screening cells' point ranges, assembly -> cross term
     T* x = coefficients + level_offsets[d];
     PSR_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));
     if (sink) sink->put("normal_load_" + std::to_string(d), loads[d].p, n, s);
@@ -1834,24 +1933,23 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
       float* msp = nullptr;
       DBuf<T> hist;
       if (tp) hist.alloc(int64_t(p.iters) * n, s);
+      auto sweep = [&](auto s_tag, auto i_tag) {
+        using S = decltype(s_tag);
+        using I = decltype(i_tag);
+        relax_strips_planned<S, T, I>(sched, L.plan, reinterpret_cast<const S*>(svals.p),
+                                      reinterpret_cast<const I*>(sidx.p), b.p, x, p.iters, s, msp, hist.p, false, false,
+                                      dp);
+      };
       if (mixed) {
         if (sched.wide)
-          relax_strips_scheduled<float, T, int32_t>(sched, reinterpret_cast<const float*>(svals.p),
-                                                    reinterpret_cast<const int32_t*>(sidx.p), b.p, x, p.iters, s, msp,
-                                                    hist.p, false, false, dp);
+          sweep(float(), int32_t());
         else
-          relax_strips_scheduled<float, T, int16_t>(sched, reinterpret_cast<const float*>(svals.p),
-                                                    reinterpret_cast<const int16_t*>(sidx.p), b.p, x, p.iters, s, msp,
-                                                    hist.p, false, false, dp);
+          sweep(float(), int16_t());
       } else {
         if (sched.wide)
-          relax_strips_scheduled<T, T, int32_t>(sched, reinterpret_cast<const T*>(svals.p),
-                                                reinterpret_cast<const int32_t*>(sidx.p), b.p, x, p.iters, s, msp,
-                                                hist.p, false, false, dp);
+          sweep(T(), int32_t());
         else
-          relax_strips_scheduled<T, T, int16_t>(sched, reinterpret_cast<const T*>(svals.p),
-                                                reinterpret_cast<const int16_t*>(sidx.p), b.p, x, p.iters, s, msp,
-                                                hist.p, false, false, dp);
+          sweep(T(), int16_t());
       }
       if (stats) {  // relax_ms and level_relax_ms are filled by stats->finish()
         stats->row_visits += n * p.iters;
@@ -1878,6 +1976,7 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
       PSR_CUDA(cudaMemcpyAsync(tp->cum[d].p, cumulative.p, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
       if (screened) tp->points[d] = std::move(P);
     }
+    L.release();
   }
   if (tp) {
     tp->pcol = std::move(pcol);
