@@ -618,7 +618,7 @@ __device__ __forceinline__ void cell_hats(const T p[3], const int cell[3], int d
 // order, same arithmetic as screening_row.
 template <class T>
 __device__ __forceinline__ double screening_row_same(const PointsView<T>& P, const int c[3], int d, uint32_t present,
-                                                     double acc[27], int2* rout) {
+                                                     double acc[27], int2* rout, bool* any = nullptr) {
   double rhs = 0.0;
 #pragma unroll
   for (int k8 = 0; k8 < 8; ++k8) {
@@ -630,6 +630,7 @@ __device__ __forceinline__ double screening_row_same(const PointsView<T>& P, con
       if (u >= 0) range = make_int2(P.bstart[u], P.bstart[u + 1]);
     }
     if (rout) rout[k8] = range;
+    if (any && range.x < range.y) *any = true;
     for (int32_t j = range.x; j < range.y; ++j) {
       T p[3] = {P.spos[3 * j], P.spos[3 * j + 1], P.spos[3 * j + 2]};
       T weight = P.sw[j];
@@ -691,8 +692,8 @@ __global__ void assemble_level_kernel(const int64_t* keys, int64_t n, int d, Col
 template <class T, class S, class I, bool SCREEN>
 __global__ void __launch_bounds__(128, 5) assemble_sliced_kernel(const int64_t* keys, int64_t n, int d, ColumnView cv, int64_t off,
                                        const double* table, PointsView<T> P, const double* load, const int32_t* inv,
-                                       const int32_t* group_off, S* svals, I* sidx, T* sb,
-                                       int2* ranges_out = nullptr) {
+                                       const int32_t* group_off, S* svals, I* sidx, T* sb, int2* ranges_out,
+                                       uint8_t* has_points) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   int c[3];
@@ -717,8 +718,10 @@ __global__ void __launch_bounds__(128, 5) assemble_sliced_kernel(const int64_t* 
 #pragma unroll
   for (int k = 0; k < 27; ++k) acc[k] = 0.0;
   double pl = 0.0;
-  if (SCREEN) pl = screening_row_same(P, c, d, present, acc, ranges_out ? ranges_out + 8 * i : nullptr);
+  bool any = false;
+  if (SCREEN) pl = screening_row_same(P, c, d, present, acc, ranges_out ? ranges_out + 8 * i : nullptr, &any);
   const int64_t p = inv[i];
+  if (has_points) has_points[p] = any;
   __align__(16) S v[28];  // written to global memory as 16-byte vectors
 #pragma unroll
   for (int k = 0; k < 27; ++k) {
@@ -1418,6 +1421,7 @@ struct SlicedTape {
   StripSchedule sched;
   DBuf<char> svals, sidx;  // schedule-order operator rows (float32 values in the mixed precision)
   DBuf<T> b;               // schedule-order right-hand side after the cross term
+  DBuf<uint8_t> has_points;  // schedule order: a point lies in one of the row's eight cells (screened levels)
   DBuf<T> hist;            // n x iters (schedule order): x after each visit
   DBuf<int32_t> ccols;     // cross operator (rows at d, columns at d-1), key order, 28 slots
   DBuf<T> cvals;
@@ -1537,6 +1541,7 @@ struct LevelPrep {
   StripPlan plan;
   DBuf<char> svals, sidx;
   DBuf<int2> cell_ranges;
+  DBuf<uint8_t> has_points;
   cudaEvent_t ready = nullptr;  // recorded on the side stream after the preparation
   // From here on the buffers belong to stream s (it waits for the preparation): they are used and
   // freed in its order.
@@ -1545,7 +1550,7 @@ struct LevelPrep {
     PSR_CUDA(cudaStreamWaitEvent(s, ready, 0));
     auto take = [s](auto&... buffer) { ((buffer.s = s), ...); };
     take(P.pos, P.w, P.spos, P.sw, P.ids, P.bstart, P.bkeys, P.bins.slots, cols, vals, b, sched.perm, sched.inv,
-         sched.off, sched.skeys, plan.xstart, plan.bounds, plan.visits, plan.meta, svals, sidx, cell_ranges);
+         sched.off, sched.skeys, plan.xstart, plan.bounds, plan.visits, plan.meta, svals, sidx, cell_ranges, has_points);
   }
   void release() { *this = LevelPrep(); }
   LevelPrep() = default;
@@ -1560,6 +1565,7 @@ struct LevelPrep {
     svals = std::move(o.svals);
     sidx = std::move(o.sidx);
     cell_ranges = std::move(o.cell_ranges);
+    has_points = std::move(o.has_points);
     std::swap(ready, o.ready);
     return *this;
   }
@@ -1730,6 +1736,7 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
       StripSchedule& sched = L.sched;
       build_strip_schedule(keys_at(d), n, d, sched, q);
       if (screened) L.cell_ranges.alloc(8 * n, q);
+      if (screened && tp) L.has_points.alloc(n, q);
       const int sbytes = mixed ? 4 : int(sizeof(T));
       const int ibytes = sched.wide ? 4 : 2;
       L.svals.alloc(kSlots * n * sbytes, q);
@@ -1749,7 +1756,7 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
           auto assemble = screened ? assemble_sliced_kernel<T, S, I, true> : assemble_sliced_kernel<T, S, I, false>;
           assemble<<<blocks_for(n, 128), 128, 0, q>>>(keys_at(d), n, d, bcv, level_offsets[d], table.p, pv,
                                                       loads[d].p, sched.inv.p, sched.off.p, sv, si, L.b.p,
-                                                      L.cell_ranges.p);
+                                                      L.cell_ranges.p, L.has_points.p);
           PSR_LAUNCH_CHECK();
         }
         plan_strips<S, T, I>(sched, p.iters, false, L.plan, q);
@@ -1967,6 +1974,7 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
         st.sched = std::move(sched);
         st.svals = std::move(svals);
         st.sidx = std::move(sidx);
+        st.has_points = std::move(L.has_points);
         st.b = std::move(b);
         st.hist = std::move(hist);
       }
