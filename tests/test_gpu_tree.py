@@ -34,3 +34,21 @@ def test_bitmap_tree_has_the_sorted_tree_s_keys(monkeypatch, depth, full_depth, 
     assert len(runs[0][1]) == len(runs[1][1]) == depth + 1
     for a, b in zip(runs[0][1], runs[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("depth,full_depth", [(10, 2), (11, 2), (12, 1)])
+def test_deep_records_match_the_oracle(dtype, depth, full_depth):
+    """32-bit record keys through depth 10 and 64-bit ones beyond, bitmap trees through depth 11
+    and sorted ones beyond: every basis key, and the density and normal fields behind them."""
+    import oracle
+    from warp_psr_b200 import reconstruct
+    P, N = _cloud(200, seed=depth)
+    p, n = P.cpu().numpy().astype(dtype), N.cpu().numpy().astype(dtype)
+    opts = dict(depth=depth, full_depth=full_depth, base_depth=1, iters=1, samples_per_node=1e-8)  # finest records
+    r = reconstruct(torch.from_numpy(p).cuda(), torch.from_numpy(n).cuda(), **opts)
+    ref = oracle.OracleResult(p, n, **opts)
+    np.testing.assert_array_equal(r.field.keys.cpu().numpy(), ref.keys)
+    tol = 2e-6 if dtype == np.float32 else 1e-13  # per stage, and 8 times it on the coefficients
+    scale = np.abs(ref.coefficients).max()
+    assert np.abs(r.field.coefficients.cpu().numpy() - ref.coefficients).max() <= 8 * tol * scale
