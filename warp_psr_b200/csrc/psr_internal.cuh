@@ -146,7 +146,8 @@ SampleGroups<T> prepare_samples(const T* pos, const T* nrm, int64_t n, int depth
 // ---------------------------------------------------------------- A2 density.py
 template <class T>
 struct DensityData {
-  std::vector<DBuf<int64_t>> agg_keys;  // per depth, sorted basis keys of occupied cells
+  // Basis keys of occupied cells per depth: sorted at the leaf depth, in morton order above it.
+  std::vector<DBuf<int64_t>> agg_keys;
   std::vector<DBuf<T>> agg_values;      // 4 per record: position sum xyz, weight
   std::vector<int64_t> agg_count;
   DBuf<T> dw;                           // 2 per group: raw splat depth, splat weight

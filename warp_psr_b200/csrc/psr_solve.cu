@@ -469,9 +469,24 @@ __global__ void points_kernel(const int64_t* keys, const T* vals, int64_t m, int
   ids[i] = int32_t(i);
 }
 
-__global__ void bin_heads_kernel(const uint64_t* keys, int64_t n, int32_t* heads) {
+// Marks the first point of every bin (`keys` sorted) and puts the bin's points in the order of
+// their cells' keys, in which the screening sums take them.  The sort leaves them in the order of
+// the aggregates, which is morton order above the leaf depth.  A bin holds several points only
+// where the means of neighbouring cells lie on (or round onto) its faces, so the insertion sort
+// of a bin by the thread of its first point has next to nothing to do.
+__global__ void bin_heads_kernel(const uint64_t* keys, int64_t n, const int64_t* cells, int32_t* ids, int32_t* heads) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i < n) heads[i] = (i == 0 || keys[i] != keys[i - 1]);
+  if (i >= n) return;
+  const bool head = i == 0 || keys[i] != keys[i - 1];
+  heads[i] = head;
+  if (!head) return;
+  for (int64_t j = i + 1; j < n && keys[j] == keys[i]; ++j) {
+    const int32_t id = ids[j];
+    const int64_t cell = cells[id];
+    int64_t k = j;
+    for (; k > i && cells[ids[k - 1]] > cell; --k) ids[k] = ids[k - 1];
+    ids[k] = id;
+  }
 }
 
 __global__ void bin_fill_kernel(const uint64_t* keys, const int32_t* heads, const int32_t* prefix, int64_t n, int d,
@@ -507,7 +522,7 @@ struct PointsView {
   const T* w = nullptr;
   const T* spos = nullptr;          // pos and w in bin order (spos[3j + a] = pos[3 ids[j] + a])
   const T* sw = nullptr;
-  const int32_t* ids = nullptr;     // point ids sorted by bin (stable)
+  const int32_t* ids = nullptr;     // point ids sorted by bin, in the order of their cells' keys inside one
   const int32_t* bstart = nullptr;  // per unique bin, start into ids; count+1 entries
   HashView bins;                    // basis key of a bin cell -> unique bin index
 };
@@ -1470,19 +1485,17 @@ static PointsData<T> make_points(const DensityData<T>& D, const NormalData<T>& N
     int Db = d > 0 ? d : 1;
     sort_pairs(bk.p, sbk.p, ids.p, P.ids.p, m, 3 * Db, s);
   }
-  P.spos.alloc(3 * m, s);
-  P.sw.alloc(m, s);
-  if (m) {
-    bin_order_points_kernel<T><<<blocks_for(m), kThreads, 0, s>>>(P.ids.p, m, P.pos.p, P.w.p, P.spos.p, P.sw.p);
-    PSR_LAUNCH_CHECK();
-  }
   // Unique bins: at most m.  The arrays and the bin hash are sized for m and the hash takes
   // the count from the device, so the count is never read back (a host synchronisation).
   DBuf<int32_t> heads(m, s), prefix(m, s);
+  P.spos.alloc(3 * m, s);
+  P.sw.alloc(m, s);
   if (m) {
-    bin_heads_kernel<<<blocks_for(m), kThreads, 0, s>>>(sbk.p, m, heads.p);
+    bin_heads_kernel<<<blocks_for(m), kThreads, 0, s>>>(sbk.p, m, D.agg_keys[d].p, P.ids.p, heads.p);
     PSR_LAUNCH_CHECK();
     inclusive_sum(heads.p, prefix.p, m, s);
+    bin_order_points_kernel<T><<<blocks_for(m), kThreads, 0, s>>>(P.ids.p, m, P.pos.p, P.w.p, P.spos.p, P.sw.p);
+    PSR_LAUNCH_CHECK();
   }
   P.nbins = m;  // an upper bound; the bins are the first prefix[m - 1] entries
   P.bkeys.alloc(m, s);
