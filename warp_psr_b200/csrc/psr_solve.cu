@@ -1543,6 +1543,31 @@ struct SideStream {
   }
 };
 
+// Device memory that the default pool could still hand out: free on the device, or held by the
+// pool and not in use.
+static int64_t available_bytes() {
+  size_t free = 0, total = 0;
+  PSR_CUDA(cudaMemGetInfo(&free, &total));
+  int dev = 0;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  PSR_CUDA(cudaGetDevice(&dev));
+  PSR_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+  PSR_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  PSR_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return int64_t(free) + int64_t(reserved) - int64_t(used);
+}
+
+// Levels prepared ahead are held together, where the chain by itself holds one at a time: without
+// a tape, which keeps every level anyway, a call's peak is a third and more higher (3.5 million
+// points at depth 10, mixed precision, 9.2 -> 10.7 GB; 100,000 with a chain of nodes down to
+// depth 11 each, 10.7 -> 14.6 GB).  So levels past this bound are only prepared ahead while all of
+// them take at most a quarter of the memory that is left (a level's temporaries are smaller than
+// what it holds), and a call that fits the device one level at a time still does.  Such a call
+// prepares its finest levels on the caller's stream, one by one: 65.5 instead of 64.5 ms at
+// depth 10.  Asking for the memory that is left is worth it past the bound only.
+constexpr int64_t kAheadBytes = int64_t(1) << 30;
+
 // One level's point constraints, operator rows, schedule and sweep plan, before the chain takes
 // them.
 template <class T>
@@ -1714,18 +1739,37 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
     tp->mixed = sizeof(T) == 8 && p.precision == 1;
   }
   const bool mixed = sizeof(T) == 8 && p.precision == 1;
-  // Point constraints, operators, schedules and sweep plans depend on no level's solution, only
-  // the chain base solve -> (cross term, sweeps, prolongation) per level does, and its coarse end
-  // leaves most of the GPU idle: the base solve runs on one CTA and the sweeps of the coarse
-  // levels on a few dozen.  So the finer levels are prepared on a stream of their own while the
-  // chain starts (a depth-8 float32 call 8.17 -> 7.48 ms, depth-9 mixed
-  // 20.7 -> 20.0 ms, 2,011 points at depth 5 2.60 -> 2.42 ms).  What a
-  // level's preparation allocates belongs to that stream until the chain has waited for the
-  // level, and to the caller's stream from then on (LevelPrep::hand_over).
+  // Point constraints, operators, schedules and sweep plans depend on no level's solution; only
+  // the chain base solve -> (cross term, sweeps, prolongation) per level does, and the base solve
+  // runs on one CTA.  So the levels above it are prepared on a stream of their own beside the
+  // base solve (a depth-8 float32 call 8.17 -> 7.48 ms, 2,011 points at depth 5 2.60 -> 2.42 ms;
+  // not beside the sweeps: a sweep plan's read-back holds the host until its level is assembled,
+  // and the chain goes on after the last of them).  What a level's preparation allocates belongs
+  // to that stream until the chain has waited for the level, and to the caller's stream from then
+  // on (LevelPrep::hand_over).
+  int ahead = base;  // the finest level prepared ahead
+  if (count_at(base)) {
+    auto held_bytes = [&](int d) {  // rows with 32-bit neighbour indices at most, points with their bins
+      const int64_t row = kSlots * (mixed ? 4 : sizeof(T)) + 32 * 4 + sizeof(T) + 16 + (screened ? 64 : 0);
+      return count_at(d) * row + (screened ? D.agg_count[d] * int64_t(8 * sizeof(T) + 80) : 0);
+    };
+    int64_t held = 0, limit = kAheadBytes;
+    const char* forced = std::getenv("PSR_AHEAD_BYTES");  // test override: what a call meets when memory is short
+    if (forced) limit = std::atoll(forced);
+    bool asked = forced || tp;
+    while (ahead < p.solve_depth && count_at(ahead + 1)) {
+      held += held_bytes(ahead + 1);
+      if (held > limit && !asked) {
+        limit = std::max(limit, available_bytes() / 4);
+        asked = true;
+      }
+      if (held > limit && (forced || !tp)) break;
+      ++ahead;
+    }
+  }
   SideStream side(s);  // outlives what is prepared on it
   std::vector<LevelPrep<T>> prepared(finest + 1);
-  const bool finer = p.solve_depth > base && count_at(base) > 0 && count_at(base + 1) > 0;
-  const cudaStream_t q_finer = finer ? side.get() : s;
+  const cudaStream_t q_ahead = ahead > base ? side.get() : s;
   auto prepare = [&](int d, cudaStream_t q) {
     const int64_t n = count_at(d);
     LevelPrep<T>& L = prepared[d];
@@ -1796,10 +1840,10 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
     int64_t n = count_at(d);
     if (!n) break;
     if (tp) tp->top = d;
-    if (d == base)
+    if (d == base || d > ahead)
       prepare(d, s);
     else if (d == base + 1)  // the base solve is under way on s
-      for (int e = d; e <= p.solve_depth && count_at(e); ++e) prepare(e, q_finer);
+      for (int e = d; e <= ahead; ++e) prepare(e, q_ahead);
     LevelPrep<T>& L = prepared[d];
     L.hand_over(s);
     PointsData<T>& P = L.P;
