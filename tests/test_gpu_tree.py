@@ -52,3 +52,24 @@ def test_deep_records_match_the_oracle(dtype, depth, full_depth):
     tol = 2e-6 if dtype == np.float32 else 1e-13  # per stage, and 8 times it on the coefficients
     scale = np.abs(ref.coefficients).max()
     assert np.abs(r.field.coefficients.cpu().numpy() - ref.coefficients).max() <= 8 * tol * scale
+
+
+@pytest.mark.parametrize("count,finest", [(5, 3), (3000, 7)])
+def test_bitmaps_reach_down_to_the_finest_records_only(count, finest):
+    """A sparse cloud at depth 11: no record lies deeper than `finest`, so the tree needs none of
+    the 321 MB of bitmaps and counts of the levels below (459 MB at the peak with them, of which
+    the dense column tables of the basis keys and the records take 85)."""
+    import ctypes
+    from warp_psr_b200 import _lib, reconstruct
+    _lib.load()
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool, used_high, word = ctypes.c_void_p(), 8, ctypes.c_uint64(0)  # cudaMemPoolAttrUsedMemHigh
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), torch.cuda.current_device()) == 0
+    P, N = _cloud(count, seed=11)
+    torch.cuda.synchronize()
+    assert rt.cudaMemPoolSetAttribute(pool, used_high, ctypes.byref(word)) == 0
+    r = reconstruct(P, N, depth=11, full_depth=2, solve_depth=2, keep_stages=True)
+    torch.cuda.synchronize()
+    assert rt.cudaMemPoolGetAttribute(pool, used_high, ctypes.byref(word)) == 0
+    assert int(r.diagnostics["stage"]("normal_keys", torch.int64).max()) >> 48 <= finest
+    assert word.value < 200 << 20

@@ -186,13 +186,18 @@ static int64_t sort_unique(DBuf<uint64_t>& keys, int64_t n, int end_bit, uint64_
 // ------------------------------------------------------------------ the tree on bitmaps
 // A brood of level d is a node of level d - 1: its coordinates lie in [-2, 2^(d-1) + 1] (the
 // dilation by one of the halved coordinates of the finer level's broods, which lie in
-// [-2, 2^d + 1], stays there).  One bit per node of that grid, rows along z padded to whole words:
-// 2.4 MB at depth 9, 18 MB at depth 10, 140 MB at depth 11.  A set is then united by OR-ing words
-// and comes out sorted and unique, so a level needs no sort of its 27 candidates per request, and
-// no count of one level is needed on the host to build the next: the whole tree waits for the
-// host once instead of twice per level.  A call with 2,011 points at depth 5:
-// 3.59 -> 2.84 ms, 200,000 at depth 8 10.2 -> 8.7, 800,000 at depth 9 24.9 -> 22.5.
-// Past depth 11 the bitmaps outgrow the sorts (1.1 GB at depth 12) and build_tree sorts.
+// [-2, 2^d + 1], stays there).  One bit per node of that grid, rows along z padded to whole words,
+// and a count per word: 5.7 MB through depth 9, 42 MB through depth 10, 321 MB through depth 11,
+// for the levels down to the finest one with records (finer levels have no broods).  A set is then
+// united by OR-ing words and comes out sorted and unique, so a level needs no sort of its 27
+// candidates per request, and no count of one level is needed on the host to build the next: the
+// whole tree waits for the host once instead of twice per level.  A call with 2,011 points at
+// depth 5: 3.59 -> 2.84 ms, 200,000 at depth 8 10.2 -> 8.7, 800,000 at depth 9 24.9 -> 22.5.
+// The tree stage against the sorts (records with the finest ones at the tree's depth, then 5 points
+// in a few coarse records): depth 8 217 and 1,661 us (730,000 records), 82 and 336; depth 10 878 and
+// 5,462 (8.6 million), 350 and 1,401 (135 records), 82 and 338; depth 11 2,354 and 8,415 (2.6
+// million), 1,500 and 1,600 (135 records), 84 and 343 (1,460 with the empty levels' bitmaps).
+// Past depth 11 the bitmaps outgrow the sorts (2.5 GB at depth 12) and build_tree sorts.
 constexpr int kBitmapDepth = 11;
 constexpr int kBitmapLow = -2;
 
@@ -369,11 +374,14 @@ static TreeData build_tree_bitmap(const NormalData<T>& N, int depth, int full_de
   tree.basis.resize(depth + 1);
   tree.support_count.assign(depth + 1, 0);
   tree.basis_count.assign(depth + 1, 0);
+  int top = full_depth;  // the finest level with broods
+  for (int d = full_depth + 1; d <= depth; ++d)
+    if (N.offsets[d + 1] > N.offsets[d]) top = d;
   BroodLevels L{};
-  L.depth = depth;
-  for (int d = 0; d <= depth; ++d) L.base[d + 1] = L.base[d] + brood_words(d);
-  for (int d = depth + 1; d <= kBitmapDepth; ++d) L.base[d + 1] = L.base[d];
-  const int64_t words = L.base[depth + 1];
+  L.depth = top;
+  for (int d = 0; d <= top; ++d) L.base[d + 1] = L.base[d] + brood_words(d);
+  for (int d = top + 1; d <= kBitmapDepth; ++d) L.base[d + 1] = L.base[d];
+  const int64_t words = L.base[top + 1];
   DBuf<uint32_t> bits(words, s);
   bits.zero();
   coarse_bits_kernel<<<blocks_for(L.base[full_depth + 1]), kThreads, 0, s>>>(L, full_depth, bits.p);
@@ -387,7 +395,7 @@ static TreeData build_tree_bitmap(const NormalData<T>& N, int depth, int full_de
   // requests of the level before, and the finer broods only add their parents.
   DBuf<uint32_t> requests;
   int requests_depth = -1;  // the level whose brood grid `requests` is on; -1: none
-  for (int d = depth - 1; d >= 0; --d) {
+  for (int d = top - 1; d >= 0; --d) {
     const uint32_t* finer = bits.p + L.base[d + 1];
     const unsigned blocks = blocks_for(brood_words(d + 1));
     if (d > base_depth) {
@@ -397,9 +405,9 @@ static TreeData build_tree_bitmap(const NormalData<T>& N, int depth, int full_de
     }
     parent_bits_kernel<<<blocks, kThreads, 0, s>>>(finer, d, 0, bits.p + L.base[d]);
     PSR_LAUNCH_CHECK();
-    // level d + 1's requests: level d + 2's broods (none at the finest level), or the last halving
+    // level d + 1's requests: level d + 2's broods (none past the finest level), or the last halving
     const bool first = d == base_depth;
-    if (first ? d + 2 > depth : requests_depth < 0) continue;
+    if (first ? d + 2 > top : requests_depth < 0) continue;
     DBuf<uint32_t> halved(brood_words(d + 1), s);
     halved.zero();
     parent_bits_kernel<<<blocks_for(brood_words(d + 2)), kThreads, 0, s>>>(first ? bits.p + L.base[d + 2] : requests.p,
@@ -410,22 +418,22 @@ static TreeData build_tree_bitmap(const NormalData<T>& N, int depth, int full_de
     requests = std::move(halved);
     requests_depth = d + 1;
   }
-  DBuf<int32_t> counts(words, s), prefix(words, s);
-  DBuf<int> totals(2 * (depth + 1), s);  // broods through each level, basis nodes of each level
+  DBuf<int32_t> prefix(words, s);  // broods of every word, summed in place
+  DBuf<int> totals(2 * (top + 1), s);  // broods through each level, basis nodes of each level
   totals.zero();
-  brood_count_kernel<<<blocks_for(words), kThreads, 0, s>>>(bits.p, L, words, counts.p, totals.p + depth + 1);
+  brood_count_kernel<<<blocks_for(words), kThreads, 0, s>>>(bits.p, L, words, prefix.p, totals.p + top + 1);
   PSR_LAUNCH_CHECK();
-  inclusive_sum(counts.p, prefix.p, words, s);
+  inclusive_sum(prefix.p, prefix.p, words, s);
   brood_totals_kernel<<<1, 32, 0, s>>>(prefix.p, L, totals.p);
   PSR_LAUNCH_CHECK();
-  const std::vector<int> total = read_vector(totals.p, 2 * (depth + 1), s);
+  const std::vector<int> total = read_vector(totals.p, 2 * (top + 1), s);
   TreeOut out{};
   int64_t broods = 0, basis = 0;
-  for (int d = 0; d <= depth; ++d) {
+  for (int d = 0; d <= top; ++d) {
     out.brood0[d] = broods;
     out.basis0[d] = basis;
     tree.support_count[d] = 8 * (total[d] - broods);
-    tree.basis_count[d] = total[depth + 1 + d];
+    tree.basis_count[d] = total[top + 1 + d];
     tree.support[d].alloc(tree.support_count[d], s);
     tree.basis[d].alloc(tree.basis_count[d], s);
     out.support[d] = tree.support[d].p;
@@ -441,7 +449,7 @@ static TreeData build_tree_bitmap(const NormalData<T>& N, int depth, int full_de
   brood_expand_kernel<<<blocks_for(broods), kThreads, 0, s>>>(list.p, broods, prefix.p, L, out, mark.p);
   PSR_LAUNCH_CHECK();
   inclusive_sum(mark.p, rank.p, 8 * broods, s);
-  brood_basis_kernel<<<blocks_for(8 * broods), kThreads, 0, s>>>(mark.p, rank.p, 8 * broods, depth, out);
+  brood_basis_kernel<<<blocks_for(8 * broods), kThreads, 0, s>>>(mark.p, rank.p, 8 * broods, top, out);
   PSR_LAUNCH_CHECK();
   return tree;
 }
