@@ -46,6 +46,20 @@ def test_footprint_beyond_every_strip_count_is_an_error(monkeypatch):
         gpu_relax(keys, offsets, columns, values, b, x, 3, 2)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("iters,limit", [(8, "1"), (19, None)])
+def test_pipelines_need_no_strip_plan(monkeypatch, dtype, iters, limit):
+    """The cluster pipelines take a level that no strip plan of the dynamic scheduler would (a
+    footprint limit of 1); where they decline (19 visits: more clusters than fit), the dynamic
+    scheduler makes its plan then."""
+    monkeypatch.setenv("PSR_RELAX_KERNEL", "pipeline")
+    if limit:
+        monkeypatch.setenv("PSR_RELAX_FOOTPRINT_LIMIT", limit)
+    keys, offsets, columns, values, b, x = local_system("random", size=33, depth=5, dtype=dtype, seed=3)
+    expected = oracle.relax_sliced(keys, 5, offsets, columns, values, b, x, iters)
+    np.testing.assert_array_equal(gpu_relax(keys, offsets, columns, values, b, x, 5, iters), expected)
+
+
 @pytest.mark.parametrize("precision", ["double", "float", "mixed"])
 @pytest.mark.parametrize("name,value", FORCED)
 def test_forced_paths_reconstruct_identically(monkeypatch, precision, name, value):

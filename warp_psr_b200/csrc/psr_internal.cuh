@@ -334,6 +334,7 @@ void build_strip_schedule(const int64_t* keys, int64_t rows, int depth, StripSch
 // memory a task takes.  Depends on the schedule, the sweeps, the types and the direction only, so
 // it can be made before the level's right-hand side is known.
 struct StripPlan {
+  // strips 0: only xstart is there (the cluster pipelines were asked for)
   int strips = 0, unstaged = 0, nvisits = 0, cap = 0, row_cap = 0, b_cap = 0;
   int64_t smem = 0;
   DBuf<int32_t> xstart, bounds;
@@ -345,7 +346,7 @@ void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cuda
 
 // relax_strips_scheduled (below) with its plan at hand.
 template <class T, class V, class I>
-void relax_strips_planned(const StripSchedule& S, const StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
+void relax_strips_planned(const StripSchedule& S, StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
                           int iters, cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment,
                           RelaxDeferred* defer);
 

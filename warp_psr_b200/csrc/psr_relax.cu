@@ -1356,6 +1356,11 @@ void throw_relax_error(int err) {
   if (err) throw Error(4, "ordered relaxation: a dependency wait timed out");
 }
 
+static bool pipeline_asked() {
+  const char* mode = std::getenv("PSR_RELAX_KERNEL");
+  return mode && std::string(mode) == "pipeline";
+}
+
 // The cluster pipelines for one level, when they apply: every task's rows fit a region and
 // its footprint, peer segments and exports fit shared memory, and `iters` clusters of
 // kPipeCtas CTAs can be resident at once.  Returns false (nothing launched) otherwise.
@@ -1365,9 +1370,7 @@ template <class T, class V, class I>
 static bool relax_pipeline(const StripSchedule& S, const T* svals, const I* sidx, const V* sb, const int32_t* xstart,
                            V* xb0, V* xb1, int iters, cudaStream_t s, float* ms, V* hist, bool rev,
                            bool record_increment, RelaxDeferred* defer) {
-  const char* mode = std::getenv("PSR_RELAX_KERNEL");
-  const bool forced = mode && std::string(mode) == "pipeline";
-  if (!forced) return false;  // opt-in: measured slower than the dynamic scheduler
+  if (!pipeline_asked()) return false;  // opt-in: measured slower than the dynamic scheduler
   const int depth = S.depth, n = 1 << depth, strips = kPipeCtas;
   const int per16 = 16 / int(sizeof(V));
   if (int64_t(iters) * kPipeCtas > device_sms()) return false;
@@ -1541,18 +1544,14 @@ static bool relax_pipeline(const StripSchedule& S, const T* svals, const I* sidx
   return true;
 }
 
+// The tasks of the dynamic scheduler; P.xstart is there.
 template <class T, class V, class I>
-void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cudaStream_t s) {
+static void plan_tasks(const StripSchedule& S, int iters, bool rev, StripPlan& P, cudaStream_t s) {
   const int64_t rows = S.rows;
-  if (iters <= 0 || rows <= 0) return;
   const int n = 1 << S.depth;
-  const int nx = n + 2;
   const int per16 = 16 / int(sizeof(V));
   const int32_t* off = S.off.p;
-  P.xstart.alloc(int64_t(n + 1) * 4 * nx, s);
-  DBuf<int32_t>& xstart = P.xstart;
-  xstart_kernel<<<blocks_for(int64_t(n + 1) * 4 * nx), kThreads, 0, s>>>(S.skeys.p, off, n, xstart.p);
-  PSR_LAUNCH_CHECK();
+  const DBuf<int32_t>& xstart = P.xstart;
   // Strips per slice: a wave (iters x strips tasks) fills about seven eighths of the persistent
   // grid, leaving CTAs that take the next wave's tasks early and prefetch their operator rows;
   // at least ~128 rows per strip.  More strips are taken (up to twice as many) while more than
@@ -1661,7 +1660,19 @@ void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cuda
 }
 
 template <class T, class V, class I>
-void relax_strips_planned(const StripSchedule& S, const StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
+void plan_strips(const StripSchedule& S, int iters, bool rev, StripPlan& P, cudaStream_t s) {
+  if (iters <= 0 || S.rows <= 0) return;
+  const int n = 1 << S.depth;
+  const int64_t entries = int64_t(n + 1) * 4 * (n + 2);
+  P.xstart.alloc(entries, s);
+  xstart_kernel<<<blocks_for(entries), kThreads, 0, s>>>(S.skeys.p, S.off.p, n, P.xstart.p);
+  PSR_LAUNCH_CHECK();
+  // The cluster pipelines make tasks of their own (and take levels that these could reject).
+  if (!pipeline_asked()) plan_tasks<T, V, I>(S, iters, rev, P, s);
+}
+
+template <class T, class V, class I>
+void relax_strips_planned(const StripSchedule& S, StripPlan& P, const T* svals, const I* sidx, const V* sb, V* x,
                           int iters, cudaStream_t s, float* ms, V* hist, bool rev, bool record_increment,
                           RelaxDeferred* defer) {
   const int64_t rows = S.rows;
@@ -1678,6 +1689,7 @@ void relax_strips_planned(const StripSchedule& S, const StripPlan& P, const T* s
     PSR_LAUNCH_CHECK();
     return;
   }
+  if (!P.strips) plan_tasks<T, V, I>(S, iters, rev, P, s);  // the pipelines declined
   const int strips = P.strips;
   DBuf<int> ctrl(2 * 32, s);  // task counter and error word: one 128-byte line each
   ctrl.zero();
@@ -1868,7 +1880,7 @@ template void relax_sliced_csr<double>(const int64_t*, int64_t, int, const int32
 namespace psr {
 #define PSR_SCHED(T, V, I)                                                                                       \
   template void plan_strips<T, V, I>(const StripSchedule&, int, bool, StripPlan&, cudaStream_t);                 \
-  template void relax_strips_planned<T, V, I>(const StripSchedule&, const StripPlan&, const T*, const I*,        \
+  template void relax_strips_planned<T, V, I>(const StripSchedule&, StripPlan&, const T*, const I*,        \
                                               const V*, V*, int, cudaStream_t, float*, V*, bool, bool,           \
                                               RelaxDeferred*);                                                   \
   template void relax_strips_scheduled<T, V, I>(const StripSchedule&, const T*, const I*, const V*, V*, int,  \
