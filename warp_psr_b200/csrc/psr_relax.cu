@@ -1729,9 +1729,7 @@ void relax_strips_planned(const StripSchedule& S, StripPlan& P, const T* svals, 
   auto kernel = rev ? strip_gs_kernel<T, V, I, true> : strip_gs_kernel<T, V, I, false>;
   PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const int64_t total_tasks = int64_t(P.nvisits) * strips;
-  // a wave's tasks and the next one's, whose rows are fetched ahead: a coarse level leaves the
-  // other SMs to the preparation of the finer ones
-  const int grid = int(std::min<int64_t>({total_tasks, int64_t(kRelaxCtasPerSm) * device_sms(), 2ll * strips * iters}));
+  const int grid = int(std::min<int64_t>(total_tasks, int64_t(kRelaxCtasPerSm) * device_sms()));
   const char* trace_file = std::getenv("PSR_RELAX_TRACE_FILE");
   DBuf<long long> trace;
   if (trace_file) {
