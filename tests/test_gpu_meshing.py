@@ -125,6 +125,22 @@ def test_grids_of_every_spacing_match_pointwise_evaluation(dtype, shape, slab):
     assert fused.metadata["retained_cells"] == generic.metadata["retained_cells"]
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("cap", [0, 160, 200, 260])
+def test_bricks_past_their_capacity_evaluate_node_by_node(monkeypatch, dtype, cap):
+    # none, 12 %, 56 % and 98 % of the bricks within the capacity (110 to 278 functions each on
+    # this grid): the same mesh
+    P, N = _sphere_cloud(3000, dtype, seed=3)
+    res = reconstruct(P, N, depth=5, full_depth=2)
+    options = dict(resolution=(71, 68, 131), bounds=_inner_bounds(P))
+    full = extract_mesh(res, **options)
+    monkeypatch.setenv("PSR_MESH_BRICK_CAP", str(cap))
+    lowered = extract_mesh(res, **options)
+    assert len(full.indices) > 1000
+    assert torch.equal(lowered.indices, full.indices)
+    assert torch.equal(lowered.vertices, full.vertices)
+
+
 def test_mesh_vertex_loss_reaches_inputs():
     """loss = sum |v|^2 over the mesh vertices; its gradient on positions and normals against
     central differences (float64, h = 1e-6), with the cell selection and connectivity checked

@@ -622,7 +622,10 @@ void slab_values(const psr_field_handle& h, const mc::Grid& g, int64_t start, in
   const double bytes = functions * (2 * sizeof(T) + 1);
   if (h.depth < mc::kMaxLevels && h.cumulative && h.hash_slots && functions <= 3.0 * b.bx * b.by * b.bz &&
       bytes <= 47 * 1024) {
-    const int cap = int(functions);
+    int cap = int(functions);
+    // PSR_MESH_BRICK_CAP lowers the functions a brick may hold (test override: bricks past the
+    // capacity, which the host's count leaves to rounding, and which evaluate node by node).
+    if (const char* env = std::getenv("PSR_MESH_BRICK_CAP")) cap = std::min(cap, std::max(std::atoi(env), 0));
     mc::brick_values_kernel<T><<<unsigned(bricks), mc::kBrickThreads, size_t(bytes), s>>>(h, g, b, start, T(iso), cap,
                                                                                           values);
   } else {
