@@ -1338,6 +1338,15 @@ static int device_smem_per_sm() {
   return bytes;
 }
 
+// Dynamic shared memory of one CTA of the sweeps, at most (the rest is their static shared memory).
+// The kernels' limit is set to it, not to a launch's own size: the limit is a property of the
+// kernel, and another thread's smaller level would lower it between this thread's setting and its
+// launch.
+static int64_t strip_smem_budget() {
+  return std::min<int64_t>(device_smem_optin(), device_smem_per_sm() / kRelaxCtasPerSm) - 4096;
+}
+static int64_t pipeline_smem_budget() { return int64_t(device_smem_optin()) - 2048; }
+
 template <class V>
 __global__ void gather_x_kernel(const int32_t* perm, int64_t n, const V* x, V* sx) {
   int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1408,7 +1417,7 @@ static bool relax_pipeline(const StripSchedule& S, const T* svals, const I* sidx
   P.cap = std::max(c[0], 1);
   P.ecap = std::max(c[3], 1);
   auto al = [](int64_t b) { return (b + 127) & ~int64_t(127); };
-  const int64_t budget = int64_t(device_smem_optin()) - 2048;  // static shared memory of the kernel
+  const int64_t budget = pipeline_smem_budget();
   {  // rows per region: all of them if they fit, else as many as fit beside the rest
     const int64_t fixed = 2 * al(int64_t(P.cap + 1) * int64_t(sizeof(V))) + 2 * al(int64_t(P.ecap) * int64_t(sizeof(V))) +
                           2 * al(int64_t(sizeof(PipeMeta))) + kPipeRegions * 3 * 128;
@@ -1457,7 +1466,7 @@ static bool relax_pipeline(const StripSchedule& S, const T* svals, const I* sidx
   }
   if (off > budget) return false;
   auto kernel = rev ? pipeline_gs_kernel<T, V, I, true> : pipeline_gs_kernel<T, V, I, false>;
-  PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(off)));
+  PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(budget)));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1585,7 +1594,7 @@ static void plan_tasks(const StripSchedule& S, int iters, bool rev, StripPlan& P
   }
   // Shared memory of one CTA: the footprint (and its +0 entry), the staged rows and their
   // right-hand sides.
-  const int64_t budget = std::min<int64_t>(device_smem_optin(), device_smem_per_sm() / kRelaxCtasPerSm) - 4096;
+  const int64_t budget = strip_smem_budget();
   const int64_t row_bytes = kSlotsR * int64_t(sizeof(T)) + kIdxSlots * int64_t(sizeof(I));
   auto fp_bytes_of = [&](int fp) { return (int64_t(std::max(fp, 1) + 1) * int64_t(sizeof(V)) + 15) & ~int64_t(15); };
   // staged rows and right-hand-side elements that fit beside a footprint of fp elements
@@ -1727,7 +1736,7 @@ void relax_strips_planned(const StripSchedule& S, StripPlan& P, const T* svals, 
   L.meta = reinterpret_cast<const StripMeta*>(P.meta.p);
   const int64_t smem = P.smem;
   auto kernel = rev ? strip_gs_kernel<T, V, I, true> : strip_gs_kernel<T, V, I, false>;
-  PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  PSR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(strip_smem_budget())));
   const int64_t total_tasks = int64_t(P.nvisits) * strips;
   const int grid = int(std::min<int64_t>(total_tasks, int64_t(kRelaxCtasPerSm) * device_sms()));
   const char* trace_file = std::getenv("PSR_RELAX_TRACE_FILE");
