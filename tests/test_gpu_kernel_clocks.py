@@ -52,3 +52,33 @@ def test_clocks_cover_forward_and_reverse(monkeypatch):
     assert fwd["bytes"] == pytest.approx(fwd["units"] * (27 * 4 + 3 * 8 + 4 + 8))
     assert fwd["launches"] == r.diagnostics["relax_launches"]
     assert _lib.kernel_clocks() == []  # read once, then cleared
+
+
+@pytest.mark.parametrize("point_weight", [0.0, 2.0])
+def test_row_adjoint_bytes_count_what_the_rows_read(monkeypatch, point_weight):
+    """level_rows_reverse_kernel: every row reads its key, position, right-hand-side adjoint and
+    cross row (12 + 8 + 28 * 12 bytes, and a flag where the level is screened) and the level adds
+    onto the coarser coefficients; only rows with a point in one of their cells -- none without
+    screening, at most eight per point with it -- gather their neighbours' visit records."""
+    monkeypatch.setenv("PSR_KERNEL_CLOCKS", "1")
+    p, n = cloud()
+    res = reconstruct_differentiable(p.clone().requires_grad_(True), n, precision="mixed",
+                                     **dict(OPTS, point_weight=point_weight))
+    v, _, _ = res.evaluate(p[:64].double(), centered=True)
+    _lib.kernel_clocks()
+    torch.nan_to_num(v).sum().backward()
+    torch.cuda.synchronize()
+    clocks = {c["kernel"]: c for c in _lib.kernel_clocks()}
+    rows = clocks["level_rows_reverse_kernel"]
+    counts = res.result.metadata["basis_counts"]
+    coarser = sum(counts[OPTS["full_depth"]:OPTS["depth"]])
+    every = rows["units"] * (12 + 8 + 28 * 12 + (point_weight > 0)) + 2 * 8 * coarser
+    gathering = (rows["bytes"] - every) / (32 * 2 + 2 * 8 * 8 + 28 * 8)
+    if point_weight == 0:
+        assert gathering == pytest.approx(0, abs=1e-6)
+    else:
+        screening = clocks["screening_points_reverse_kernel"]
+        points = screening["units"]
+        assert screening["bytes"] == pytest.approx(points * 8 * 8 + gathering * 28 * 8 + 8 * coarser)
+        assert gathering == pytest.approx(round(gathering), abs=1e-6)
+        assert points < gathering < min(8 * points, rows["units"])

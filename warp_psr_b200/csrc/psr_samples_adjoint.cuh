@@ -9,7 +9,7 @@ __device__ __forceinline__ void quadratic_grad(double x, double g[3]) {
   g[2] = x;
 }
 
-// Normal splat (normal_splat_kernel) and the weighted average (average_contrib_kernel /
+// Normal splat (normal_groups_kernel, normal_reduce_kernel) and the weighted average (average_contrib_kernel /
 // average_finish_kernel) reversed, one group per thread in first-index order.
 template <class T>
 __global__ void normal_splat_reverse_kernel(const int32_t* order, int64_t n, const T* sums, const T* nsums,

@@ -290,14 +290,24 @@ __global__ void level_reverse_kernel(LevelReverse<T, S, I> L) {
   }
 }
 
+// Flags set among n (for the byte model of a clocked launch: waits for the host).
+static int64_t count_flags(const uint8_t* flags, int64_t n, cudaStream_t s) {
+  DBuf<int32_t> sum(1, s);
+  size_t temp = 0;
+  PSR_CUDA(cub::DeviceReduce::Sum(nullptr, temp, flags, sum.p, n, s));
+  DBuf<char> t(int64_t(temp), s);
+  PSR_CUDA(cub::DeviceReduce::Sum(t.p, temp, flags, sum.p, n, s));
+  return read_scalar(sum.p, s);
+}
+
 // The per-row pass of a sliced level with the stored cross operator, unrolled so that every
 // per-slot quantity stays in registers: the operator adjoint of the row (written to row_gA,
 // 28 per row, for the per-point screening pass) and -C^T g_b into the coarser cumulative.
 // Only the screening pass reads operator adjoints, and only those of rows with a point in one
 // of their eight cells (has_points): the other rows -- and all rows of an unscreened level --
 // skip the gathers of their neighbours' visit records, which are most of the pass.  Bound by
-// those gathers (L2) and the scattered rows written.  Solve and adjoint of a depth-9
-// scan 40.1 -> 39.0 ms, at depth 10 130.1 -> 125.2 ms.
+// those gathers (L2) and the scattered rows written.  The launches of a depth-9 scan's five levels
+// 3.00 -> 1.95 ms, of a depth-10 scan's 9.96 -> 7.26 ms (rows of 28 in 16-byte stores included).
 template <class T, class I, int ITERS>
 __global__ void __launch_bounds__(128) level_rows_reverse_kernel(const int64_t* __restrict__ skeys, int64_t n,
                                                                  const int32_t* __restrict__ perm,
@@ -1195,15 +1205,20 @@ void solve_backward(void* tape_ptr, const TreeData& tree, const DensityData<T>& 
         rA.alloc(kSlots * n, s);
         L.row_gA = rA.p;
       }
-      // per row: sorted key, permutation, index row, reverse and forward visit records, g_b,
-      // the 27 operator adjoints, the cross tape row; the coarser cumulative adjoint read and
-      // written
+      // per row: sorted key, permutation, g_b, the cross tape row; per row whose operator adjoint
+      // is made: index row, reverse and forward visit records, the adjoint row; the coarser
+      // cumulative adjoint read and written
+      const bool rows_pass = p.iters == 8 && L.ccols;
+      int64_t marked = 0;  // rows whose operator adjoint is read
+      if (tp.screened && kernel_clocks_on()) marked = count_flags(st.has_points.p, n, s);
+      const int64_t gathering = rows_pass ? marked : n;
       KernelClock rows_clock(kClkLevelRowsReverse,
-                             n * (8.0 + 4 + 32 * sizeof(I) + 2.0 * p.iters * sizeof(T) + sizeof(T) +
-                                  (tp.screened ? 27 * sizeof(T) : 0) + kSlots * (4.0 + sizeof(T))) +
+                             n * (8.0 + 4 + sizeof(T) + kSlots * (4.0 + sizeof(T)) + (tp.screened ? 1 : 0)) +
+                                 gathering * (32.0 * sizeof(I) + 2.0 * p.iters * sizeof(T) +
+                                              (tp.screened ? kSlots * sizeof(T) : 0)) +
                                  2.0 * count_at(d - 1) * sizeof(T),
                              double(n), s);
-      if (p.iters == 8 && L.ccols) {
+      if (rows_pass) {
         level_rows_reverse_kernel<T, I, 8><<<blocks_for(n, 128), 128, 0, s>>>(
             st.sched.skeys.p, n, st.sched.perm.p, L.off, L.sidx, L.xhist, L.mu, L.g_b, L.ccols, L.cvals,
             L.g_cum_prev, st.has_points.p, tp.screened ? rA.p : nullptr);
@@ -1214,10 +1229,10 @@ void solve_backward(void* tape_ptr, const TreeData& tree, const DensityData<T>& 
       rows_clock.stop();
       if (tp.screened && tp.points[d].m) {
         const int64_t m = tp.points[d].m;
-        // per point: position and weight read, their adjoints written; per row: g_b and the
-        // 27 operator adjoints; the coarser cumulative solution
+        // per point: position and weight read, their adjoints written; per row with a point in one
+        // of its cells: g_b and the 27 operator adjoints; the coarser cumulative solution
         KernelClock points_clock(kClkScreeningReverse,
-                                 m * 8.0 * sizeof(T) + n * 28.0 * sizeof(T) + count_at(d - 1) * double(sizeof(T)),
+                                 m * 8.0 * sizeof(T) + marked * 28.0 * sizeof(T) + count_at(d - 1) * double(sizeof(T)),
                                  double(m), s);
         screening_points_reverse_kernel<T><<<blocks_for(m, 128), 128, 0, s>>>(
             L.P, m, d, bcv, level_offsets[d], g_b.p, rA.p, kSlots, tp.cum[d - 1].p, level_offsets[d - 1], g_pos[d].p,
