@@ -21,6 +21,11 @@ struct Error : std::runtime_error {
   Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
 
+// Device memory ran out (a call that holds more than it must can do with less).
+struct OutOfMemory : Error {
+  explicit OutOfMemory(const std::string& m) : Error(2, m) {}
+};
+
 #define PSR_CUDA(call)                                                                              \
   do {                                                                                              \
     cudaError_t e_ = (call);                                                                        \
@@ -62,7 +67,17 @@ struct DBuf {
     release();
     s = stream;
     n = count;
-    if (count > 0) PSR_CUDA(cudaMallocAsync((void**)&p, size_t(count) * sizeof(T), stream));
+    if (count > 0) {
+      const cudaError_t e = cudaMallocAsync((void**)&p, size_t(count) * sizeof(T), stream);
+      if (e == cudaErrorMemoryAllocation) {
+        p = nullptr;
+        n = 0;
+        cudaGetLastError();  // no later launch's error
+        throw OutOfMemory("cudaMallocAsync of " + std::to_string(count * int64_t(sizeof(T))) +
+                          " bytes: " + cudaGetErrorString(e));
+      }
+      PSR_CUDA(e);
+    }
   }
   void zero() {
     if (n > 0) PSR_CUDA(cudaMemsetAsync(p, 0, size_t(n) * sizeof(T), s));

@@ -228,6 +228,13 @@ struct SolveStats {
     release();
     throw_relax_error(err);
   }
+  void restart() {  // nothing counted or timed yet
+    release();
+    relax_ms = 0;
+    row_visits = launches = finest_row_visits = 0;
+    level_relax_ms.clear();
+    if (relax_error.p) relax_error.zero();
+  }
   void release() {
     for (auto& e : relax_events) {
       cudaEventDestroy(e.first);

@@ -1543,30 +1543,16 @@ struct SideStream {
   }
 };
 
-// Device memory that the default pool could still hand out: free on the device, or held by the
-// pool and not in use.
-static int64_t available_bytes() {
-  size_t free = 0, total = 0;
-  PSR_CUDA(cudaMemGetInfo(&free, &total));
-  int dev = 0;
-  cudaMemPool_t pool;
-  uint64_t reserved = 0, used = 0;
-  PSR_CUDA(cudaGetDevice(&dev));
-  PSR_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
-  PSR_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
-  PSR_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-  return int64_t(free) + int64_t(reserved) - int64_t(used);
-}
-
 // Levels prepared ahead are held together, where the chain by itself holds one at a time: without
 // a tape, which keeps every level anyway, a call's peak is a third and more higher (3.5 million
 // points at depth 10, mixed precision, 9.2 -> 10.7 GB; 100,000 with a chain of nodes down to
-// depth 11 each, 10.7 -> 14.6 GB).  So levels past this bound are only prepared ahead while all of
-// them take at most a quarter of the memory that is left (a level's temporaries are smaller than
-// what it holds), and a call that fits the device one level at a time still does.  Such a call
-// prepares its finest levels on the caller's stream, one by one: 65.5 instead of 64.5 ms at
-// depth 10.  Asking for the memory that is left is worth it past the bound only.
-constexpr int64_t kAheadBytes = int64_t(1) << 30;
+// depth 11 each, 10.7 -> 14.6 GB).  So levels past this bound (a twentieth of the device's memory,
+// everything up to some four million points) are prepared on the caller's stream when the chain
+// reaches them (no level ahead: 66.4 instead of 64.5 ms at depth 10).  A call that still runs out of
+// memory is solved again with no level prepared ahead, so what fits the device one level at a time
+// runs.  The memory that is left is not asked for: cudaMemGetInfo takes 70 us, and 2 to 60 ms where
+// other processes keep the driver busy.
+constexpr int64_t kAheadBytes = int64_t(8) << 30;
 
 // One level's point constraints, operator rows, schedule and sweep plan, before the chain takes
 // them.
@@ -1612,11 +1598,14 @@ struct LevelPrep {
   }
 };
 
+// solve_levels (below) once; `together` in: levels may be prepared ahead, out: some are.
 template <class T>
-void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalData<T>& N,
-                  const std::vector<int64_t>& level_offsets, const int64_t* all_keys, const HashMap& all_hash,
-                  const Params& p, T* coefficients, cudaStream_t s, SolveStats* stats, StageSink* sink,
-                  std::shared_ptr<void>* tape_out) {
+static void solve_once(const TreeData& tree, const DensityData<T>& D, const NormalData<T>& N,
+                       const std::vector<int64_t>& level_offsets, const int64_t* all_keys, const HashMap& all_hash,
+                       const Params& p, T* coefficients, cudaStream_t s, SolveStats* stats, StageSink* sink,
+                       std::shared_ptr<void>* tape_out, bool& together) {
+  const bool may_prepare_ahead = together;
+  together = false;
   const int finest = p.depth, base = p.base_depth;
   std::shared_ptr<SolveTape<T>> tape_holder;
   SolveTape<T>* tp = nullptr;
@@ -1742,37 +1731,34 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
   // Point constraints, operators, schedules and sweep plans depend on no level's solution; only
   // the chain base solve -> (cross term, sweeps, prolongation) per level does, and the base solve
   // runs on one CTA.  So the levels above it are prepared on a stream of their own beside the
-  // base solve (a depth-8 float32 call 8.17 -> 7.48 ms, 2,011 points at depth 5 2.60 -> 2.42 ms;
-  // not beside the sweeps: a sweep plan's read-back holds the host until its level is assembled,
-  // and the chain goes on after the last of them).  What a level's preparation allocates belongs
-  // to that stream until the chain has waited for the level, and to the caller's stream from then
-  // on (LevelPrep::hand_over).
+  // base solve (a depth-8 float32 call 8.25 -> 7.41 ms, 2,011 points at depth 5 2.72 -> 2.49 ms,
+  // depth-9 mixed 21.6 -> 20.8 ms; not beside the sweeps: a sweep plan's read-back holds the host
+  // until its level is assembled, and the chain goes on after the last of them).  What a level's
+  // preparation allocates belongs to that stream until the chain has waited for the level, and to
+  // the caller's stream from then on (LevelPrep::hand_over).
   int ahead = base;  // the finest level prepared ahead
   if (count_at(base)) {
     auto held_bytes = [&](int d) {  // rows with 32-bit neighbour indices at most, points with their bins
       const int64_t row = kSlots * (mixed ? 4 : sizeof(T)) + 32 * 4 + sizeof(T) + 16 + (screened ? 64 : 0);
       return count_at(d) * row + (screened ? D.agg_count[d] * int64_t(8 * sizeof(T) + 80) : 0);
     };
-    int64_t held = 0, limit = kAheadBytes;
-    const char* forced = std::getenv("PSR_AHEAD_BYTES");  // test override: what a call meets when memory is short
-    if (forced) limit = std::atoll(forced);
-    bool asked = forced || tp;
-    while (ahead < p.solve_depth && count_at(ahead + 1)) {
+    int64_t held = 0, limit = tp ? std::numeric_limits<int64_t>::max() : kAheadBytes;
+    if (const char* env = std::getenv("PSR_AHEAD_BYTES")) limit = std::atoll(env);  // test override
+    while (may_prepare_ahead && ahead < p.solve_depth && count_at(ahead + 1)) {
       held += held_bytes(ahead + 1);
-      if (held > limit && !asked) {
-        limit = std::max(limit, available_bytes() / 4);
-        asked = true;
-      }
-      if (held > limit && (forced || !tp)) break;
+      if (held > limit) break;
       ++ahead;
     }
   }
+  together = ahead > base;
   SideStream side(s);  // outlives what is prepared on it
   std::vector<LevelPrep<T>> prepared(finest + 1);
   const cudaStream_t q_ahead = ahead > base ? side.get() : s;
   auto prepare = [&](int d, cudaStream_t q) {
     const int64_t n = count_at(d);
     LevelPrep<T>& L = prepared[d];
+    if (const char* env = std::getenv("PSR_AHEAD_FAIL"))  // test override: no memory for this level ahead
+      if (q != s && std::atoi(env) == d) throw OutOfMemory("PSR_AHEAD_FAIL");
     if (screened) L.P = make_points(D, N, bh, d, p.point_weight, bool(p.exact), q);
     const PointsView<T> pv = screened ? L.P.view() : PointsView<T>();
     const int res = 1 << d;
@@ -2047,6 +2033,25 @@ void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalDat
     tp->pcol = std::move(pcol);
     tp->pval = std::move(pval);
   }
+}
+
+template <class T>
+void solve_levels(const TreeData& tree, const DensityData<T>& D, const NormalData<T>& N,
+                  const std::vector<int64_t>& level_offsets, const int64_t* all_keys, const HashMap& all_hash,
+                  const Params& p, T* coefficients, cudaStream_t s, SolveStats* stats, StageSink* sink,
+                  std::shared_ptr<void>* tape_out) {
+  bool together = true;
+  try {
+    solve_once(tree, D, N, level_offsets, all_keys, all_hash, p, coefficients, s, stats, sink, tape_out, together);
+    return;
+  } catch (const OutOfMemory&) {
+    if (!together) throw;
+  }
+  if (tape_out) tape_out->reset();
+  PSR_CUDA(cudaStreamSynchronize(s));  // what the attempt held is free
+  if (stats) stats->restart();
+  together = false;
+  solve_once(tree, D, N, level_offsets, all_keys, all_hash, p, coefficients, s, stats, sink, tape_out, together);
 }
 
 template void solve_levels<float>(const TreeData&, const DensityData<float>&, const NormalData<float>&,
